@@ -90,6 +90,7 @@ lt_status make_queue_item(lt_context *ctx, const lt_request *r, int precision, d
     }
     const bool c32 = precision == LT_FP32C;
     a.recs = cat->recs;
+    a.nie = nie_of(cat);
     a.chunks = r->kmap ? cat->chunks_k : cat->chunks;
     a.nchunks = r->kmap ? cat->nchunks_k : cat->nchunks;
     a.kmap = r->kmap ? 1 : 0;
@@ -107,7 +108,7 @@ lt_status make_queue_item(lt_context *ctx, const lt_request *r, int precision, d
     a.scale = r->scale;
     a.status = ctx->status;
     it->op = op;
-    it->ppt = c32 ? (ppt32 == 1 ? 1 : 2) : ((op & OP_POT) ? 1 : 2);
+    it->ppt = c32 && ppt32 == 1 ? 1 : 2;
     const int P = it->ppt;
     a.tiles_x = (a.nx + 32 * P - 1) / (32 * P);
     a.ntiles = a.tiles_x * ((a.ny + 7) / 8);
@@ -117,7 +118,6 @@ lt_status make_queue_item(lt_context *ctx, const lt_request *r, int precision, d
         it->recs32 = fc.recs32;
         it->chunks32 = fc.chunks;
         it->nchunks32 = cat->nhalos ? fc.nchunks : 0;
-        it->nie64 = fc.nie;
         it->mu_tol = det ? kMuTol32 : 0.0;
     }
     if (cat->nhalos == 0) a.nchunks = 0;

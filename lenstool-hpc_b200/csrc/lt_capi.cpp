@@ -259,14 +259,8 @@ lt_status lt_create(int device, size_t budget, lt_context **out)
      * catalogue */
     for (int p = 0; p < 3; p++)
         for (int o = 0; o < 8; o++) ctx->shape[p][o] = LT_SHAPE(2, 1);
-    ctx->shape[LT_FP64][OP_HESS] = LT_SHAPE(2, 2);
-    ctx->shape[LT_FP64][OP_POT] = LT_SHAPE(1, 2);
-    ctx->shape[LT_FP64][OP_HESS | OP_POT] = LT_SHAPE(1, 2);
-    ctx->shape[LT_FP64][OP_GRAD] = LT_SHAPE(2, 2);
-    ctx->shape[LT_FP64_FAST][OP_HESS] = LT_SHAPE(2, 2);
-    ctx->shape[LT_FP64_FAST][OP_POT] = LT_SHAPE(1, 2);
-    ctx->shape[LT_FP64_FAST][OP_HESS | OP_POT] = LT_SHAPE(1, 2);
-    ctx->shape[LT_FP64_FAST][OP_GRAD] = LT_SHAPE(2, 2);
+    for (int p : {(int)LT_FP64, (int)LT_FP64_FAST})
+        for (int o : {(int)OP_GRAD, (int)OP_HESS, (int)OP_POT, OP_HESS | OP_POT}) ctx->shape[p][o] = LT_SHAPE(2, 2);
     ctx->shape[LT_FP32C][OP_HESS] = LT_SHAPE4(2, 2, 256, 128);
     ctx->shape[LT_FP32C][OP_POT] = LT_SHAPE4(2, 2, 256, 128);
     ctx->shape[LT_FP32C][OP_HESS | OP_POT] = LT_SHAPE4(2, 2, 256, 128);
@@ -490,6 +484,7 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
     GridArgs a;
     memset(&a, 0, sizeof(a));
     a.recs = cat->recs;
+    a.nie = nie_of(cat);
     a.chunks = kmap ? cat->chunks_k : cat->chunks;
     a.nchunks = kmap ? cat->nchunks_k : cat->nchunks;
     a.kmap = kmap;
@@ -522,17 +517,22 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
             count_launch(1);
             return launch_epilogue_zero(b, ctx->num_sms, s);
         }
-        if (precision == LT_FP64) {
-            /* the Hessian with the reference's rounding sequence, the potential through its
-             * pi05 formula */
-            const int xop = ((op & OP_HESS) ? ((op & ~OP_HESS) | OP_HEX) : op) | ((op & OP_POT) ? OP_PEX : 0);
-            return launch_grid64_tiled(xop, b, ctx->num_sms, s, ctx->shape[LT_FP64][op & 7]);
+        if (precision == LT_FP64 && (op & OP_HESS)) {
+            /* the Hessian with the reference's rounding sequence; with the potential (its
+             * own records and registers) as two launches, each writing its planes */
+            const int n = b.nout;
+            int pot = n;
+            if (op & OP_POT)
+                for (pot = 0; pot < n && b.kinds[pot] != KIND_POT;) pot++;
+            b.nout = pot;
+            int err = launch_grid64_tiled(OP_HEX, b, ctx->num_sms, s, ctx->shape[LT_FP64][op & 7]);
+            if (err != cudaSuccess || pot == n) return err;
+            b.nout = 1;
+            b.kinds[0] = KIND_POT;
+            b.out[0] = b.out[pot];
+            return launch_grid64_tiled(OP_POT, b, ctx->num_sms, s, ctx->shape[LT_FP64][OP_POT]);
         }
-        if (precision == LT_FP64_FAST) {
-            /* the dPIE deflection as log(1 + eps) (a deflection-only call: no kernel combines it) */
-            const int fop = op == OP_GRAD ? (OP_GRAD | OP_GFX) : op;
-            return launch_grid64_tiled(fop, b, ctx->num_sms, s, ctx->shape[LT_FP64_FAST][op & 7]);
-        }
+        if (precision != LT_FP32C) return launch_grid64_tiled(op, b, ctx->num_sms, s, ctx->shape[precision][op & 7]);
         return launch_fp32c(ctx, cat, op, b, s);
     };
     if (!host) {

@@ -40,15 +40,15 @@ constexpr int kHitCap = 64;             /* delensing hits recorded per source */
 /* ---- step 2: sources ------------------------------------------------------------- */
 
 template <int TYPE>
-__device__ __forceinline__ void grad_run(const lt_rec64 *recs, int start, int count, double x, double y, double &gx,
+__device__ __forceinline__ void grad_run(const lt_nie64 *recs, int start, int count, double x, double y, double &gx,
                                          double &gy)
 {
-    for (int h = start; h < start + count; h++) grad_pair<TYPE>(recs[h], x, y, gx, gy);
+    for (int h = start; h < start + count; h++) grad_nie<TYPE>(recs[h], nie64<TYPE>(recs[h], x, y), gx, gy);
 }
 
 /* One block per system, one thread per image: the deflection at the image over every
  * halo (chunk order, as the grid kernel), then thread 0 forms the barycentre. */
-__global__ void chi2_sources_kernel(Chi2Dev c, const lt_rec64 *recs, const lt_chunk *chunks, int nchunks)
+__global__ void chi2_sources_kernel(Chi2Dev c, const lt_nie64 *recs, const lt_chunk *chunks, int nchunks)
 {
     __shared__ double sx[kMaxImg * 2], sy[kMaxImg * 2];
     const int s = blockIdx.x;
@@ -388,7 +388,7 @@ lt_status check_systems(lt_context *ctx, const lt_image_systems *sys)
 static int chi2_steps(lt_context *ctx, const lt_catalog *cat, const Chi2Dev &c, bool sources_given, cudaStream_t s)
 {
     if (!sources_given) {
-        chi2_sources_kernel<<<c.nsys, 64, 0, s>>>(c, cat->recs, cat->chunks, cat->nhalos ? cat->nchunks : 0);
+        chi2_sources_kernel<<<c.nsys, 64, 0, s>>>(c, nie_of(cat), cat->chunks, cat->nhalos ? cat->nchunks : 0);
         count_launch(1);
     } else {
         cudaMemsetAsync(c.hits, 0, 4 * (size_t)c.nsys, s);
@@ -412,6 +412,7 @@ int chi2_launch(lt_context *ctx, const lt_catalog *cat, Chi2Buf &b, bool sources
     GridArgs a;
     memset(&a, 0, sizeof(a));
     a.recs = cat->recs;
+    a.nie = nie_of(cat);
     a.chunks = cat->chunks;
     a.nchunks = cat->nchunks;
     a.xmin = c.xmin;
@@ -436,11 +437,8 @@ int chi2_launch(lt_context *ctx, const lt_catalog *cat, Chi2Buf &b, bool sources
         if (err == cudaSuccess) err = (int)cudaMemsetAsync((void *)c.ay, 0, 8 * (size_t)c.n * c.n, s);
     } else if (precision == LT_FP32C) {
         err = launch_fp32c(ctx, cat, OP_GRAD, a, s);
-    } else if (precision == LT_FP64_FAST) {
-        /* the dPIE deflection as log(1 + eps), as the LT_FP64_FAST grid calls take it */
-        err = launch_grid64_tiled(OP_GRAD | OP_GFX, a, ctx->num_sms, s, ctx->shape[LT_FP64_FAST][OP_GRAD]);
     } else {
-        err = launch_grid64_tiled(OP_GRAD, a, ctx->num_sms, s, ctx->shape[LT_FP64][OP_GRAD]);
+        err = launch_grid64_tiled(OP_GRAD, a, ctx->num_sms, s, ctx->shape[precision][OP_GRAD]);
     }
     if (err != cudaSuccess) return err;
     (void)link;

@@ -9,6 +9,7 @@
 #pragma once
 #include "lt_bulk.cuh"
 #include "lt_profiles32.cuh"
+#include "lt_closed64.cuh"
 #include "lt_profiles64.cuh"
 
 namespace lt {
@@ -21,30 +22,50 @@ struct Acc64 {
     ex::Mat run[P], tot[P]; /* OP_HEX: the reference's per-run and total sums */
 };
 
+/* One staged chunk: lt_rec64 records for OP_HEX, lt_nie64 otherwise (then acc.hxx, hyy and hxy
+ * hold the convergence and shear sums until close64). */
 template <int OP, int P, int TYPE>
-__device__ __forceinline__ void eval_chunk64(const lt_rec64 *recs, int count, const double (&px)[P], double py,
+__device__ __forceinline__ void eval_chunk64(const void *staged, int count, const double (&px)[P], double py,
                                              int kmap, Acc64<OP, P> &acc)
 {
 #pragma unroll 1
     for (int h = 0; h < count; h++) {
-        const lt_rec64 &r = recs[h];
-        const double w = kmap ? r.w : 1.0;
+        if (OP & OP_HEX) {
+            const lt_rec64 &r = static_cast<const lt_rec64 *>(staged)[h];
 #pragma unroll
-        for (int k = 0; k < P; k++) {
-            if ((OP & OP_GRAD) && (OP & OP_GFX)) grad_pair_fast<TYPE>(r, px[k], py, acc.gx[k], acc.gy[k]);
-            if ((OP & OP_GRAD) && !(OP & OP_GFX)) grad_pair<TYPE>(r, px[k], py, acc.gx[k], acc.gy[k]);
-            if (OP & OP_HESS) {
-                Hess64 hh = {acc.hxx[k], acc.hyy[k], acc.hxy[k]};
-                hess_pair<TYPE>(r, px[k], py, w, hh);
-                acc.hxx[k] = hh.xx;
-                acc.hyy[k] = hh.yy;
-                acc.hxy[k] = hh.xy;
+            for (int k = 0; k < P; k++) ex::hess_pair<TYPE>(r, px[k], py, acc.run[k]);
+        } else {
+            const lt_nie64 &r = static_cast<const lt_nie64 *>(staged)[h];
+            const double w = kmap ? r.w : 1.0;
+#pragma unroll
+            for (int k = 0; k < P; k++) {
+                const Nie64 n = nie64<TYPE>(r, px[k], py);
+                if (OP & OP_GRAD) grad_nie<TYPE>(r, n, acc.gx[k], acc.gy[k]);
+                if (OP & OP_HESS) kg_nie<TYPE>(r, n, w, acc.hxx[k], acc.hyy[k], acc.hxy[k]);
+                if (OP & OP_POT) pot_nie<TYPE>(r, n, acc.psi[k]);
             }
-            if (OP & OP_HEX) ex::hess_pair<TYPE>(r, px[k], py, acc.run[k]);
-            if ((OP & OP_POT) && (OP & OP_PEX)) pot_pair<TYPE>(r, px[k], py, acc.psi[k]);
-            if ((OP & OP_POT) && !(OP & OP_PEX)) pot_pair_fast<TYPE>(r, px[k], py, acc.psi[k]);
         }
     }
+}
+
+/* eval_chunk64 over one staged chunk of any profile type. */
+template <int OP, int P>
+__device__ __forceinline__ void eval_any64(const lt_chunk &c, const void *staged, const double (&px)[P], double py,
+                                           int kmap, Acc64<OP, P> &acc)
+{
+    switch (c.type) {
+    case 81: eval_chunk64<OP, P, 81>(staged, c.count, px, py, kmap, acc); break;
+    case 8: eval_chunk64<OP, P, 8>(staged, c.count, px, py, kmap, acc); break;
+    case 5: eval_chunk64<OP, P, 5>(staged, c.count, px, py, kmap, acc); break;
+    default: break;
+    }
+}
+
+/* The records a chunk of OP is staged from. */
+template <int OP>
+__device__ __forceinline__ const void *recs_of(const GridArgs &a, int start)
+{
+    return (OP & OP_HEX) ? (const void *)(a.recs + start) : (const void *)(a.nie + start);
 }
 
 /* The FP64 recomputation's sums: convergence and sky-frame shear from the closed form
@@ -121,6 +142,21 @@ __device__ __forceinline__ void close_run64(Acc64<OP, P> &acc, int kmap, double 
             t.d = ex::A(t.d, r.d);
         }
         acc.run[k].a = acc.run[k].b = acc.run[k].c = acc.run[k].d = 0.;
+    }
+}
+
+/* A pixel's Hessian from its sums (d: the reference's d entry, equal to hxy up to rounding). */
+template <int OP, int P>
+__device__ __forceinline__ void close64(Acc64<OP, P> &acc, int k, double &d)
+{
+    if (OP & OP_HEX) {
+        acc.hxx[k] = acc.tot[k].a;
+        acc.hxy[k] = acc.tot[k].b;
+        acc.hyy[k] = acc.tot[k].c;
+        d = acc.tot[k].d;
+    } else {
+        if (OP & OP_HESS) nie_hessian(acc.hxx[k], acc.hyy[k], acc.hxy[k], acc.hxx[k], acc.hyy[k], acc.hxy[k]);
+        d = acc.hxy[k];
     }
 }
 
@@ -236,9 +272,11 @@ __device__ __forceinline__ uint64_t near_mask(const lt_rec32 *recs, int count, c
     return (uint64_t)m[0] | ((uint64_t)m[1] << 32);
 }
 
+/* One staged chunk of FP64-class halos; nie: the closed-form records of the same halos (global
+ * memory: every lane reads the same record, and such halos are few). */
 template <int OP, int P, int TYPE>
-__device__ __forceinline__ void eval64_chunk(const lt_rec64 *recs, int count, const double (&px)[P], double py, int kmap,
-                                             Acc32<P> &acc)
+__device__ __forceinline__ void eval64_chunk(const lt_rec64 *recs, const lt_nie64 *nie, int count, const double (&px)[P],
+                                             double py, int kmap, Acc32<P> &acc)
 {
 #pragma unroll 1
     for (int h = 0; h < count; h++) {
@@ -247,9 +285,9 @@ __device__ __forceinline__ void eval64_chunk(const lt_rec64 *recs, int count, co
 #pragma unroll
         for (int k = 0; k < P; k++) {
             if (OP & OP_HESS) add_hess64(acc, k, hess_term<TYPE>(r, px[k], py, w));
-            if (OP & OP_POT) acc.psi[k] = __dadd_rn(acc.psi[k], pot_term<TYPE>(r, px[k], py));
+            if (OP & OP_POT) acc.psi[k] = __dadd_rn(acc.psi[k], pot_term<TYPE>(nie[h], px[k], py));
             if (OP & OP_GRAD) {
-                const double2 t = grad_term<TYPE>(r, px[k], py);
+                const double2 t = grad_term<TYPE>(nie[h], px[k], py);
                 acc.gx[k] = __dadd_rn(acc.gx[k], t.x);
                 acc.gy[k] = __dadd_rn(acc.gy[k], t.y);
             }
@@ -261,7 +299,7 @@ __device__ __forceinline__ void eval64_chunk(const lt_rec64 *recs, int count, co
  * pixels (ix .. ix + P - 1, iy) of grid `a`.  Every record of an FP32C chunk has the same
  * Kmap weight. */
 template <int OP, int P, int TYPE>
-__device__ __forceinline__ void eval32_chunk(const lt_rec32 *recs, const lt_rec64 *recs64, int count,
+__device__ __forceinline__ void eval32_chunk(const lt_rec32 *recs, const lt_rec64 *recs64, const lt_nie64 *nie, int count,
                                              const double (&px)[P], double py, const GridArgs &a, int ix, int iy,
                                              Acc32<P> &acc)
 {
@@ -292,16 +330,17 @@ __device__ __forceinline__ void eval32_chunk(const lt_rec32 *recs, const lt_rec6
             }
             if (near) {
                 const lt_rec64 &r64 = recs64[r.idx64];
+                const lt_nie64 &rn = nie[r.idx64];
                 const double w = kmap ? r64.w : 1.0;
 #pragma unroll
                 for (int k = 0; k < P; k++) {
                     if (OP & OP_HESS) add_hess64(acc, k, hess_term<TYPE>(r64, px[k], py, w));
                     if (OP & OP_GRAD) {
-                        const double2 t = grad_term<TYPE>(r64, px[k], py);
+                        const double2 t = grad_term<TYPE>(rn, px[k], py);
                         acc.gx[k] = __dadd_rn(acc.gx[k], t.x);
                         acc.gy[k] = __dadd_rn(acc.gy[k], t.y);
                     }
-                    if (OP & OP_POT) acc.psi[k] = __dadd_rn(acc.psi[k], pot_term<TYPE>(r64, px[k], py));
+                    if (OP & OP_POT) acc.psi[k] = __dadd_rn(acc.psi[k], pot_term<TYPE>(rn, px[k], py));
                 }
             } else {
 #pragma unroll

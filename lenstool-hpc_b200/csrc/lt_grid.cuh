@@ -15,21 +15,18 @@ enum {
     KIND_POT = 102     /* potential * scale */
 };
 
-/* which sums a kernel evaluates; OP_HEX is the Hessian with the reference's rounding
- * sequence (LT_FP64), OP_HESS the reformulated one (LT_FP64_FAST and the FP32C path);
- * OP_PEX with OP_POT takes the potential through the reference's pi05 formula (LT_FP64),
- * OP_POT alone through the deflection (LT_FP64_FAST, FP32C's FP64 halos); OP_GFX with
- * OP_GRAD takes the dPIE deflection as log(1 + eps) (LT_FP64_FAST; FP32C's FP64 terms
- * always do), OP_GRAD alone in the reference's two-logarithm form (LT_FP64, the queue's
- * exact tiles, the chi2 points); OP_NI with OP_HESS takes the Hessian from the FP64
- * closed-form records lt_nie64 (nie_kg64: the FP32C path's FP64 recomputation) */
-enum { OP_GRAD = 1, OP_HESS = 2, OP_POT = 4, OP_HEX = 8, OP_PEX = 16, OP_GFX = 32, OP_NI = 64 };
+/* which sums a kernel evaluates.  OP_HEX is the Hessian with the reference's rounding
+ * sequence (LT_FP64, records lt_rec64); every other FP64 sum takes the closed forms of the
+ * records lt_nie64 (lt_closed64.cuh; OP_NI with OP_HESS is nie_kg64, the FP32C path's FP64
+ * recomputation) */
+enum { OP_GRAD = 1, OP_HESS = 2, OP_POT = 4, OP_HEX = 8, OP_NI = 16 };
 
 /* chunk.pad bits: FP32 records (FP32C list), last chunk of a run */
 enum { CHUNK_FP32 = 1, CHUNK_RUN_END = 2 };
 
 struct GridArgs {
     const lt_rec64 *recs;
+    const lt_nie64 *nie;    /* the closed-form records of the same halos */
     const lt_chunk *chunks;
     int32_t nchunks;
     int32_t kmap;

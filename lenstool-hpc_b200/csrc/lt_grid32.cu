@@ -218,17 +218,17 @@ __global__ void __launch_bounds__(NT, MINB) grid32c_kernel(const C32Args A)
         if (c.pad & CHUNK_FP32) {
             const lt_rec32 *recs = reinterpret_cast<const lt_rec32 *>(buf);
             switch (c.type) {
-            case 81: eval32_chunk<OP, P, 81>(recs, a.recs, c.count, px, py, a, ix, iy, acc); break;
-            case 8: eval32_chunk<OP, P, 8>(recs, a.recs, c.count, px, py, a, ix, iy, acc); break;
-            case 5: eval32_chunk<OP, P, 5>(recs, a.recs, c.count, px, py, a, ix, iy, acc); break;
+            case 81: eval32_chunk<OP, P, 81>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc); break;
+            case 8: eval32_chunk<OP, P, 8>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc); break;
+            case 5: eval32_chunk<OP, P, 5>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc); break;
             default: break;
             }
         } else {
             const lt_rec64 *recs = reinterpret_cast<const lt_rec64 *>(buf);
             switch (c.type) {
-            case 81: eval64_chunk<OP, P, 81>(recs, c.count, px, py, a.kmap, acc); break;
-            case 8: eval64_chunk<OP, P, 8>(recs, c.count, px, py, a.kmap, acc); break;
-            case 5: eval64_chunk<OP, P, 5>(recs, c.count, px, py, a.kmap, acc); break;
+            case 81: eval64_chunk<OP, P, 81>(recs, a.nie + c.start, c.count, px, py, a.kmap, acc); break;
+            case 8: eval64_chunk<OP, P, 8>(recs, a.nie + c.start, c.count, px, py, a.kmap, acc); break;
+            case 5: eval64_chunk<OP, P, 5>(recs, a.nie + c.start, c.count, px, py, a.kmap, acc); break;
             default: break;
             }
         }
@@ -417,7 +417,6 @@ int launch_fp32c(lt_context *ctx, const lt_catalog *cat, int op, GridArgs &a, vo
     r.list = A.list;
     r.list_count = A.list_count;
     r.list_cap = A.list_cap;
-    r.recs = reinterpret_cast<const lt_rec64 *>(fc.nie); /* the closed-form FP64 records */
     err = launch_grid64_list(OP_HESS, r, ctx->num_sms, stream);
     count_launch(1);
     pass_mark(ctx, s, 2);
@@ -452,7 +451,6 @@ int launch_fp32c_with_list(lt_context *ctx, const lt_catalog *cat, GridArgs &a, 
     r.list = A.list;
     r.list_count = A.list_count;
     r.list_cap = A.list_cap;
-    r.recs = reinterpret_cast<const lt_rec64 *>(fc.nie); /* the closed-form FP64 records */
     err = launch_grid64_list(OP_HESS, r, ctx->num_sms, stream);
     count_launch(1);
     return err;

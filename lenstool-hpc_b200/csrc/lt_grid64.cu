@@ -28,8 +28,8 @@ __global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a
     static_assert(!LIST || (OP == (OP_HESS | OP_NI)), "list mode: the FP64 recomputation's Hessian");
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(8) uint64_t bars[2];
-    lt_rec64 *buf0 = reinterpret_cast<lt_rec64 *>(smem);
-    lt_rec64 *buf1 = buf0 + LT_CHUNK;
+    unsigned char *buf0 = smem;
+    unsigned char *buf1 = smem + LT_CHUNK * sizeof(lt_rec64);
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
@@ -60,12 +60,12 @@ __global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a
 
     auto issue = [&](long s) {
         const lt_chunk c = a.chunks[s % a.nchunks];
-        lt_rec64 *dst = (s & 1) ? buf1 : buf0;
+        unsigned char *dst = (s & 1) ? buf1 : buf0;
         uint64_t *bar = &bars[s & 1];
         uint32_t bytes = (uint32_t)c.count * (uint32_t)sizeof(lt_rec64);
         fence_proxy_async_smem();
         mbar_arrive_expect_tx(bar, bytes);
-        bulk_g2s(dst, a.recs + c.start, bytes, bar);
+        bulk_g2s(dst, recs_of<OP>(a, c.start), bytes, bar);
     };
     if (tid == 0) issue(0);
 
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a
         if (b) phase1 ^= 1; else phase0 ^= 1;
 
         const lt_chunk c = a.chunks[ci];
-        const lt_rec64 *recs = b ? buf1 : buf0;
+        const unsigned char *recs = b ? buf1 : buf0;
         if (LIST) {
             /* the staged records are the closed-form records lt_nie64; acc.hxx, acc.hyy and
              * acc.hxy hold the convergence and shear sums */
@@ -140,31 +140,22 @@ __global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a
             __syncthreads(); /* buffer b is refilled by the copy issued at step s + 1 */
             continue;
         }
-        switch (c.type) {
-        case 81: eval_chunk64<OP, P, 81>(recs, c.count, px, py, a.kmap, acc); break;
-        case 8: eval_chunk64<OP, P, 8>(recs, c.count, px, py, a.kmap, acc); break;
-        case 5: eval_chunk64<OP, P, 5>(recs, c.count, px, py, a.kmap, acc); break;
-        default: break;
-        }
-        if ((OP & OP_HEX) && (c.pad & CHUNK_RUN_END)) close_run64<OP, P>(acc, a.kmap, recs[c.count - 1].w);
+        eval_any64<OP, P>(c, recs, px, py, a.kmap, acc);
+        if ((OP & OP_HEX) && (c.pad & CHUNK_RUN_END))
+            close_run64<OP, P>(acc, a.kmap, reinterpret_cast<const lt_rec64 *>(recs)[c.count - 1].w);
 
         if (ci == a.nchunks - 1 && iy < a.ny) {
             const long row = (long)iy * a.nx;
             const bool full = a.vec_ok && (ix + P <= a.nx);
-            if (OP & OP_HEX) {
+            double hyx[P];
 #pragma unroll
-                for (int k = 0; k < P; k++) {
-                    acc.hxx[k] = acc.tot[k].a;
-                    acc.hxy[k] = acc.tot[k].b;
-                    acc.hyy[k] = acc.tot[k].c;
-                }
-            }
+            for (int k = 0; k < P; k++) close64<OP, P>(acc, k, hyx[k]);
             for (int o = 0; o < a.nout; o++) {
                 double v[P];
 #pragma unroll
                 for (int k = 0; k < P; k++)
-                    v[k] = map_value4(a.kinds[o], acc.gx[k], acc.gy[k], acc.hxx[k], acc.hyy[k], acc.hxy[k],
-                                      (OP & OP_HEX) ? acc.tot[k].d : acc.hxy[k], acc.psi[k], a.D, a.mult, a.scale);
+                    v[k] = map_value4(a.kinds[o], acc.gx[k], acc.gy[k], acc.hxx[k], acc.hyy[k], acc.hxy[k], hyx[k],
+                                      acc.psi[k], a.D, a.mult, a.scale);
                 double *dst = a.out[o] + row + ix;
                 if (P == 2 && full) {
                     *reinterpret_cast<double2 *>(dst) = make_double2(v[0], v[1 % P]);
@@ -219,13 +210,10 @@ int launch_grid64(int op, const GridArgs &args, int num_sms, void *stream, bool 
     }
     switch (op) {
     case OP_GRAD: return launch_shape<OP_GRAD>(shape, args, num_sms, s);
-    case OP_GRAD | OP_GFX: return launch_shape<OP_GRAD | OP_GFX>(shape, args, num_sms, s);
     case OP_HESS: return launch_shape<OP_HESS>(shape, args, num_sms, s);
     case OP_POT: return launch_shape<OP_POT>(shape, args, num_sms, s);
     case OP_HESS | OP_POT: return launch_shape<OP_HESS | OP_POT>(shape, args, num_sms, s);
     case OP_HEX: return launch_shape<OP_HEX>(shape, args, num_sms, s);
-    case OP_POT | OP_PEX: return launch_shape<OP_POT | OP_PEX>(shape, args, num_sms, s);
-    case OP_HEX | OP_POT | OP_PEX: return launch_shape<OP_HEX | OP_POT | OP_PEX>(shape, args, num_sms, s);
     default: return (int)cudaErrorInvalidValue;
     }
 }

@@ -45,19 +45,20 @@ struct alignas(16) lt_rec64 {
 };
 static_assert(sizeof(lt_rec64) == 256, "record size");
 
-/* The FP64 record of the closed-form Hessian (the real-valued forms of
- * lt_profiles32.cuh in FP64: q = (1-e)/(1+e), s = (1+e) r, K = b0 (1-e) t05 / 2), used by
- * the FP32C path's FP64 recomputation.  Same size as lt_rec64 so that the FP64 chunk
- * lists and staging serve both.  A type-5 (SIS) record uses q2 = 1 - e, k = 1 + e,
- * K = b0 (1-e)(1+e). */
+/* The FP64 record of the closed forms (the real-valued forms of lt_profiles32.cuh in FP64:
+ * q = (1-e)/(1+e), s = (1+e) r, K = A/2 = b0 (1-e) t05 / 2, k = sqrt(1 - q^2)), used by
+ * every FP64 sum except the reference-order Hessian.  Same size as lt_rec64 so that the
+ * FP64 chunk lists and staging serve both.  A type-5 (SIS) record uses q2 = 1 - e,
+ * k = 1 + e, K = b0 (1-e)(1+e), Ak = b0. */
 struct alignas(16) lt_nie64 {
     double x0, y0, cs, sn;
     double c2t, s2t, w, k;
     double q2, sc, st, ds;
     double q2sc2, q2st2, dq2s2, opsc2;
     double opst2, opds2, tsc, tst;
-    double K, Kc1sc2, Kc1st2, pad0;
-    double pad[8];
+    double K, Kc1sc2, Kc1st2, dsq2; /* dsq2 = q^2 (s_c - s_t)                        */
+    double q2sc, q2st, qsc, qst;    /* q^2 s, q s of both radii                      */
+    double frc2, frt2, Ak, hAk;     /* 4 rc^2, 4 rcut^2, A/k and half of it          */
 };
 static_assert(sizeof(lt_nie64) == sizeof(lt_rec64), "record size");
 

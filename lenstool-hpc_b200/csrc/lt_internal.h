@@ -69,8 +69,14 @@ struct Fp32cCatalog {
     int32_t n32;
     int32_t *idx32;  /* per halo: its FP32 record, or -1 for an FP64-class halo (device) */
     int32_t *types;  /* per halo profile type (device) */
-    lt_nie64 *nie;   /* per halo (upload order): the FP64 closed-form record of the recomputation */
+    lt_nie64 *nie;   /* per halo (upload order): the FP64 closed-form record */
 };
+
+/* the closed-form records of a catalogue (device) */
+inline const lt_nie64 *nie_of(const lt_catalog *cat)
+{
+    return reinterpret_cast<const Fp32cCatalog *>(&cat->aux_desc)->nie;
+}
 
 void count_launch(uint64_t n);
 /* With pass timing on, record mark `which` (0: before pass 1, 1: after it, 2: after

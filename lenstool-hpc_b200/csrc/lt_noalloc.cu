@@ -104,6 +104,7 @@ extern "C" lt_status lt_hessian_maps_noalloc(lt_context *ctx, const lt_catalog *
     GridArgs a;
     memset(&a, 0, sizeof(a));
     a.recs = cat->recs;
+    a.nie = nie_of(cat);
     a.chunks = kmap ? cat->chunks_k : cat->chunks;
     a.nchunks = kmap ? cat->nchunks_k : cat->nchunks;
     a.kmap = kmap ? 1 : 0;

@@ -238,6 +238,7 @@ LT_HD inline void pack_nie64(const lt_rec64 &r, int type, lt_nie64 &o)
         o.q2 = sub(1., e);
         o.k = add(1., e);
         o.K = mul(mul(r.b0, sub(1., e)), add(1., e));
+        o.Ak = r.b0;
         return;
     }
     const double ope = add(1., e), ome = sub(1., e);
@@ -263,6 +264,15 @@ LT_HD inline void pack_nie64(const lt_rec64 &r, int type, lt_nie64 &o)
     o.K = K;
     o.Kc1sc2 = mul(mul(K, c1), sc2);
     o.Kc1st2 = mul(mul(K, c1), st2);
+    o.dsq2 = mul(q2, sub(sc, st));
+    o.q2sc = mul(q2, sc);
+    o.q2st = mul(q2, st);
+    o.qsc = mul(q, sc);
+    o.qst = mul(q, st);
+    o.frc2 = mul(4., mul(r.rc, r.rc));
+    o.frt2 = mul(4., mul(r.rcut, r.rcut));
+    o.hAk = div(K, o.k);
+    o.Ak = mul(2., o.hAk);
 }
 
 } // namespace pk

@@ -120,6 +120,8 @@ __device__ __forceinline__ bool walk_chunks(Stage &st, const lt_chunk *chunks, i
 }
 
 __device__ __forceinline__ bool is_grad_kind(int k) { return k == KIND_GRAD_X || k == KIND_GRAD_Y; }
+/* the sums an output kind needs */
+__device__ __forceinline__ int op_of_kind(int k) { return is_grad_kind(k) ? OP_GRAD : k == KIND_POT ? OP_POT : OP_HESS; }
 
 /* Pixel of this thread in tile `tile` (same layout as the single-grid kernels). */
 template <int P>
@@ -134,8 +136,7 @@ __device__ __forceinline__ void tile_pixel(const GridArgs &a, int tile, int &ix,
 }
 
 /* FP64 sums of one tile (grid64_kernel's per-tile work): deflection, the reference-order
- * Hessian (OP_HEX) or the fast one (OP_HESS), potential.  Writes the output planes of
- * the deflection kinds when OP is OP_GRAD, the others otherwise. */
+ * Hessian (OP_HEX) or the potential, and the output planes that need them. */
 template <int OP, int P>
 __device__ __noinline__ bool tile64(const QItem &it, int tile, Stage &st, int32_t *status)
 {
@@ -152,38 +153,28 @@ __device__ __noinline__ bool tile64(const QItem &it, int tile, Stage &st, int32_
         acc.run[k].a = acc.run[k].b = acc.run[k].c = acc.run[k].d = 0.;
         acc.tot[k].a = acc.tot[k].b = acc.tot[k].c = acc.tot[k].d = 0.;
     }
-    const bool ok = walk_chunks(st, a.chunks, a.nchunks, a.recs, nullptr, status,
-                                [&](const lt_chunk &c, const unsigned char *buf) {
-                                    const lt_rec64 *recs = reinterpret_cast<const lt_rec64 *>(buf);
-                                    switch (c.type) {
-                                    case 81: eval_chunk64<OP, P, 81>(recs, c.count, px, py, a.kmap, acc); break;
-                                    case 8: eval_chunk64<OP, P, 8>(recs, c.count, px, py, a.kmap, acc); break;
-                                    case 5: eval_chunk64<OP, P, 5>(recs, c.count, px, py, a.kmap, acc); break;
-                                    default: break;
-                                    }
+    const bool ok = walk_chunks(st, a.chunks, a.nchunks, static_cast<const lt_rec64 *>(recs_of<OP>(a, 0)), nullptr,
+                                status, [&](const lt_chunk &c, const unsigned char *buf) {
+                                    eval_any64<OP, P>(c, buf, px, py, a.kmap, acc);
                                     if ((OP & OP_HEX) && (c.pad & CHUNK_RUN_END))
-                                        close_run64<OP, P>(acc, a.kmap, recs[c.count - 1].w);
+                                        close_run64<OP, P>(acc, a.kmap,
+                                                           reinterpret_cast<const lt_rec64 *>(buf)[c.count - 1].w);
                                 });
     if (!ok) return false;
     if (iy < a.ny) {
         const long row = (long)iy * a.nx;
         const bool full = a.vec_ok && (ix + P <= a.nx);
-        if (OP & OP_HEX) {
+        double hyx[P];
 #pragma unroll
-            for (int k = 0; k < P; k++) {
-                acc.hxx[k] = acc.tot[k].a;
-                acc.hxy[k] = acc.tot[k].b;
-                acc.hyy[k] = acc.tot[k].c;
-            }
-        }
+        for (int k = 0; k < P; k++) close64<OP, P>(acc, k, hyx[k]);
         for (int o = 0; o < a.nout; o++) {
             const int kind = a.kinds[o];
-            if (is_grad_kind(kind) != (OP == OP_GRAD)) continue;
+            if (op_of_kind(kind) != (OP == OP_HEX ? (int)OP_HESS : OP)) continue;
             double v[P];
 #pragma unroll
             for (int k = 0; k < P; k++)
-                v[k] = map_value4(kind, acc.gx[k], acc.gy[k], acc.hxx[k], acc.hyy[k], acc.hxy[k],
-                                  (OP & OP_HEX) ? acc.tot[k].d : acc.hxy[k], acc.psi[k], a.D, a.mult, a.scale);
+                v[k] = map_value4(kind, acc.gx[k], acc.gy[k], acc.hxx[k], acc.hyy[k], acc.hxy[k], hyx[k], acc.psi[k], a.D,
+                                  a.mult, a.scale);
             double *dst = a.out[o] + row + ix;
             if (P == 2 && full) {
                 *reinterpret_cast<double2 *>(dst) = make_double2(v[0], v[1 % P]);
@@ -221,22 +212,22 @@ __device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_
                                   const lt_rec32 *recs = reinterpret_cast<const lt_rec32 *>(buf);
                                   switch (c.type) {
                                   case 81:
-                                      eval32_chunk<OP, P, 81>(recs, a.recs, c.count, px, py, a, ix, iy, acc);
+                                      eval32_chunk<OP, P, 81>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
                                       break;
                                   case 8:
-                                      eval32_chunk<OP, P, 8>(recs, a.recs, c.count, px, py, a, ix, iy, acc);
+                                      eval32_chunk<OP, P, 8>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
                                       break;
                                   case 5:
-                                      eval32_chunk<OP, P, 5>(recs, a.recs, c.count, px, py, a, ix, iy, acc);
+                                      eval32_chunk<OP, P, 5>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
                                       break;
                                   default: break;
                                   }
                               } else {
                                   const lt_rec64 *recs = reinterpret_cast<const lt_rec64 *>(buf);
                                   switch (c.type) {
-                                  case 81: eval64_chunk<OP, P, 81>(recs, c.count, px, py, a.kmap, acc); break;
-                                  case 8: eval64_chunk<OP, P, 8>(recs, c.count, px, py, a.kmap, acc); break;
-                                  case 5: eval64_chunk<OP, P, 5>(recs, c.count, px, py, a.kmap, acc); break;
+                                  case 81: eval64_chunk<OP, P, 81>(recs, a.nie + c.start, c.count, px, py, a.kmap, acc); break;
+                                  case 8: eval64_chunk<OP, P, 8>(recs, a.nie + c.start, c.count, px, py, a.kmap, acc); break;
+                                  case 5: eval64_chunk<OP, P, 5>(recs, a.nie + c.start, c.count, px, py, a.kmap, acc); break;
                                   default: break;
                                   }
                               }
@@ -311,7 +302,7 @@ __device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_
     }
     const bool one = !__any_sync(0xffffffffu, P == 2 && have[P - 1]); /* warp-uniform */
     double px1[1] = {qpx[0]}, py1[1] = {qpy[0]}, kap1[1] = {0.}, g11[1] = {0.}, g21[1] = {0.};
-    const bool ok2 = walk_chunks(st, a.chunks, a.nchunks, reinterpret_cast<const lt_rec64 *>(it.nie64), nullptr,
+    const bool ok2 = walk_chunks(st, a.chunks, a.nchunks, static_cast<const lt_rec64 *>(recs_of<OP_NI>(a, 0)), nullptr,
                                  status, [&](const lt_chunk &c, const unsigned char *buf) {
                                      if (!have[0]) return;
                                      const lt_nie64 *recs = reinterpret_cast<const lt_nie64 *>(buf);
@@ -467,22 +458,17 @@ __global__ void __launch_bounds__(kQThreads, MINB) queue_kernel(const QArgs q)
         }
         __syncthreads();
         bool ok = true;
-        const int hp = item.op & (OP_HESS | OP_POT);
         if (MODE == QMODE_C32) {
+            const int hp = item.op & (OP_HESS | OP_POT);
             if (item.op & OP_GRAD) ok = tile32<OP_GRAD, P32>(item, tile, st, q.status, s_list, &s_count);
             if (ok && hp == OP_HESS) ok = tile32<OP_HESS, P32>(item, tile, st, q.status, s_list, &s_count);
             if (ok && hp == OP_POT) ok = tile32<OP_POT, P32>(item, tile, st, q.status, s_list, &s_count);
             if (ok && hp == (OP_HESS | OP_POT))
                 ok = tile32<OP_HESS | OP_POT, P32>(item, tile, st, q.status, s_list, &s_count);
-        } else if (item.ppt == 2) { /* requests without the potential */
-            if (item.op & OP_GRAD) ok = tile64<OP_GRAD, 2>(item, tile, st, q.status);
-            if (ok && hp == OP_HESS) ok = tile64<OP_HEX, 2>(item, tile, st, q.status);
         } else {
-            if (item.op & OP_GRAD) ok = tile64<OP_GRAD, 1>(item, tile, st, q.status);
-            if (ok && hp == OP_HESS) ok = tile64<OP_HEX, 1>(item, tile, st, q.status);
-            if (ok && hp == OP_POT) ok = tile64<OP_POT | OP_PEX, 1>(item, tile, st, q.status);
-            if (ok && hp == (OP_HESS | OP_POT))
-                ok = tile64<OP_HEX | OP_POT | OP_PEX, 1>(item, tile, st, q.status);
+            if (item.op & OP_GRAD) ok = tile64<OP_GRAD, 2>(item, tile, st, q.status);
+            if (ok && (item.op & OP_HESS)) ok = tile64<OP_HEX, 2>(item, tile, st, q.status);
+            if (ok && (item.op & OP_POT)) ok = tile64<OP_POT, 2>(item, tile, st, q.status);
         }
         __syncthreads();
         if (!ok) break; /* a bounded wait gave up; the status word says so */

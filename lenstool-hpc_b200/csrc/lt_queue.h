@@ -13,13 +13,12 @@ struct lt_rec32;
 
 namespace lt {
 
-/* kernel modes: FP32C tiles (P = 2), or the LT_FP64 tiles with the reference-order
- * Hessian (P per request) */
+/* kernel modes: FP32C tiles, or the LT_FP64 tiles with the reference-order Hessian (P = 2) */
 enum { QMODE_C32 = 0, QMODE_EXACT = 1 };
 
 /* One request: one grid of output planes over one catalogue. */
 struct alignas(16) QItem {
-    GridArgs g;                 /* FP64 records and chunk list (the Kmap list when kmap),
+    GridArgs g;                 /* FP64 records (both kinds) and chunk list (the Kmap list when kmap),
                                    geometry (tiles_x, ntiles for this request's P),
                                    outputs, D, mult, scale, status */
     const lt_rec32 *recs32;     /* FP32C records */
@@ -28,12 +27,11 @@ struct alignas(16) QItem {
     int32_t op;                 /* OP_GRAD | OP_HESS | OP_POT */
     int32_t ntiles;
     uint32_t seq;               /* request sequence number (low 32 bits) */
-    int32_t ppt;                /* pixels per thread of the tiles (QMODE_EXACT) */
+    int32_t ppt;                /* pixels per thread of the tiles */
     int32_t pad0;
     double mu_tol;              /* FP32C: recompute pixels whose FP32 error bound on mu exceeds
                                    this in FP64 (0: none) */
     uint32_t *host_flag;        /* mapped host word set to seq + 1 on completion, or null */
-    const lt_nie64 *nie64;      /* FP32C: the closed-form FP64 records of the recomputation */
 };
 static_assert(sizeof(QItem) % 16 == 0, "QItem is copied in 16-byte units");
 
