@@ -32,8 +32,7 @@ __device__ __forceinline__ void eval_chunk64(const void *staged, int count, cons
     for (int h = 0; h < count; h++) {
         if (OP & OP_HEX) {
             const lt_rec64 &r = static_cast<const lt_rec64 *>(staged)[h];
-#pragma unroll
-            for (int k = 0; k < P; k++) ex::hess_pair<TYPE>(r, px[k], py, acc.run[k]);
+            ex::hess_pairs<TYPE, P>(r, px, py, acc.run);
         } else {
             const lt_nie64 &r = static_cast<const lt_nie64 *>(staged)[h];
             const double w = kmap ? r.w : 1.0;

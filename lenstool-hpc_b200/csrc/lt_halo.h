@@ -10,19 +10,13 @@
  *
  * Meaning of the slots by profile type
  *   type 81 (cut dPIE) and 8 (PIEMD):
- *     sqe2 = 2 sqrt(eps), cx1 = (1-eps)/(1+eps), cx1inv = 1/cx1,
- *     cxro_inv = 1/(1+eps)^2, cyro_inv = 1/(1-eps)^2, k4 = 4 eps,
- *     ci = (1-eps^2)/(2 sqrt(eps)),
- *     pref_g = ci * b0 * rcut/(rcut - rc)  (81) | ci * b0  (8)      -- deflection
- *     pref_h = ci * b0 * rcut/(rcut - rc)  (81) | ci * b0  (8)      -- Hessian, potential
- *     rc2 = rc^2, rcut2 = rcut^2, tsr_c = 2 rc sqrt(eps), tsr_t = 2 rcut sqrt(eps),
- *     e1 = 2 sqrt(eps)/(1-eps), e2 = 2 sqrt(eps)/(1+eps),
- *     dr2 = rc^2 - rcut^2, drs = rc - rcut, om2 = (1-eps)^2, e4cxi = 4 eps/(1+eps)^2,
- *     ok3c = (1-eps)(3+eps) rc, ok3t = (1-eps)(3+eps) rcut, i4rc2 = 1/(4 rc^2),
- *     i4rcut2 = 1/(4 rcut^2)  (the deflection-based potential of lt_profiles64.cuh)
- *   type 5 (SIS): cx1 = 1-eps, cx1inv = 1+eps, pref_g = (1-eps) b0,
- *     pref_h = (1+eps) b0, ci = b0 (1-eps)(1+eps)
- *   all: w = dlsds (Kmap weight), type in `type`.
+ *     sqe2 = 2 sqrt(eps), cx1 = (1-eps)/(1+eps), cx1inv = 1/cx1, cx1sq = cx1^2,
+ *     cxro = (1+eps)^2, cyro = (1-eps)^2 and their reciprocals, k4 = 4 eps,
+ *     ci = (1-eps^2)/(2 sqrt(eps)), t05 = rcut/(rcut - rc),
+ *     pref_h = ci * b0 * t05  (81) | ci * b0  (8),
+ *     rc2 = rc^2, rcut2 = rcut^2, tsr_c = 2 rc sqrt(eps), tsr_t = 2 rcut sqrt(eps)
+ *   type 5 (SIS): cx1 = 1-eps, cx1inv = 1+eps, ci = b0 (1-eps)(1+eps)
+ *   all: w = dlsds (Kmap weight)
  */
 #pragma once
 #include <stdint.h>
@@ -37,11 +31,10 @@ struct alignas(16) lt_rec64 {
     double x0, y0, cs, sn;
     double b0, eps, rc, rcut;
     double sqe2, cx1, cx1inv, cxro_inv;
-    double cyro_inv, ci, pref_g, pref_h;
+    double cyro_inv, ci, pad0, pref_h;
     double rc2, rcut2, tsr_c, tsr_t;
-    double e1, e2, w, k4;
-    double dr2, drs, om2, e4cxi;
-    double ok3c, ok3t, i4rc2, i4rcut2;
+    double w, k4, cxro, cyro;
+    double cx1sq, t05, pad[6];
 };
 static_assert(sizeof(lt_rec64) == 256, "record size");
 

@@ -74,8 +74,6 @@ LT_HD inline void pack64(int t, double x, double y, double cs, double sn, double
     if (t == 5) {
         r.cx1 = sub(1., e);
         r.cx1inv = add(1., e);
-        r.pref_g = mul(sub(1., e), b0);
-        r.pref_h = mul(add(1., e), b0);
         r.ci = mul(mul(b0, sub(1., e)), add(1., e));
         return;
     }
@@ -83,27 +81,19 @@ LT_HD inline void pack64(int t, double x, double y, double cs, double sn, double
     r.sqe2 = mul(2., sqe);
     r.cx1 = div(sub(1., e), add(1., e));
     r.cx1inv = div(1., r.cx1);
-    r.cxro_inv = div(1., mul(add(1., e), add(1., e)));
-    r.cyro_inv = div(1., mul(sub(1., e), sub(1., e)));
+    r.cx1sq = mul(r.cx1, r.cx1);
+    r.cxro = mul(add(1., e), add(1., e));
+    r.cyro = mul(sub(1., e), sub(1., e));
+    r.cxro_inv = div(1., r.cxro);
+    r.cyro_inv = div(1., r.cyro);
     r.k4 = mul(4., e);
     r.ci = div(mul(0.5, sub(1., mul(e, e))), sqe);
-    const double t05 = (t == 81) ? div(rcut, sub(rcut, rc)) : 1.0;
-    r.pref_g = mul(mul(r.ci, b0), t05);
-    r.pref_h = mul(mul(r.ci, b0), t05);
+    r.t05 = (t == 81) ? div(rcut, sub(rcut, rc)) : 1.0;
+    r.pref_h = mul(mul(r.ci, b0), r.t05);
     r.rc2 = mul(rc, rc);
     r.rcut2 = mul(rcut, rcut);
     r.tsr_c = mul(mul(2., rc), sqe);
     r.tsr_t = mul(mul(2., rcut), sqe);
-    r.e1 = div(mul(2., sqe), sub(1, e));
-    r.e2 = div(mul(2., sqe), add(1, e));
-    r.dr2 = mul(sub(rc, rcut), add(rc, rcut));
-    r.drs = sub(rc, rcut);
-    r.om2 = mul(sub(1., e), sub(1., e));
-    r.e4cxi = div(mul(4., e), mul(add(1., e), add(1., e)));
-    r.ok3c = mul(mul(sub(1., e), add(3., e)), rc);
-    r.ok3t = mul(mul(sub(1., e), add(3., e)), rcut);
-    r.i4rc2 = div(1., mul(4., mul(rc, rc)));
-    r.i4rcut2 = div(1., mul(4., mul(rcut, rcut)));
 }
 
 /* module_readParameters_calculatePotentialparameter_SOA (src/module_readParameters.cpp:

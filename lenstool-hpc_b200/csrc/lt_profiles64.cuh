@@ -145,7 +145,7 @@ struct Mat {
     double a, b, c, d;
 };
 
-/* mdci05_hpc, src/gradient2.cpp:54-83 */
+/* mdci05_hpc, src/gradient2.cpp:54-83, by IEEE division and square root */
 __device__ __forceinline__ Mat mdci05(double x, double y, double eps, double rc, double b0)
 {
     const double sqe = R(eps);
@@ -175,6 +175,114 @@ __device__ __forceinline__ Mat mdci05(double x, double y, double eps, double rc,
     return r;
 }
 
+/* Correctly rounded quotients that share a divisor (P. Markstein, "Computation of elementary
+ * functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): with
+ * y = RN(1/b), q = RN(a y) and the exact remainder r = a - q b, RN(q + r y) = RN(a/b).  Three
+ * operations a division instead of an IEEE division sequence each; the reference form divides
+ * three times by den1, three times by wrem and twice by den2 per radius.
+ *   rcp_rn: rcp64 is within half an ulp and 2^-7; one more Newton step gives RN(1/b) unless
+ *     b's significand is all ones.
+ *   sqrt_rn: from y within an ulp of 1/sqrt(x), two remainder steps give w = RN(sqrt(x)) and
+ *     RN(1/w), unless w's significand is all ones (x's then ends in 11..10 or 11..11).
+ * tests/test_hess_exact.py repeats these steps on every operand of small precisions.  The
+ * operands they do not cover (those, and values near the ends of the exponent range, where a
+ * remainder is not exact) are found by `odd_operand` and go through mdci05. */
+__device__ __forceinline__ double quot(double a, double b, double y)
+{
+    const double q = M(a, y);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+__device__ __forceinline__ double rcp_rn(double b)
+{
+    const double y = rcp64(b);
+    return __fma_rn(__fma_rn(-b, y, 1.), y, y);
+}
+/* y/2 for a normal y, off the FP64 pipe */
+__device__ __forceinline__ double half_of(double y)
+{
+    return __hiloint2double(__double2hiint(y) - 0x100000, __double2loint(y));
+}
+__device__ __forceinline__ void sqrt_rn(double x, double &w, double &iw)
+{
+    const double y = rsqrt64(x);
+    const double g = M(x, y);
+    const double g1 = __fma_rn(__fma_rn(-g, g, x), half_of(y), g);
+    const double y1 = __fma_rn(__fma_rn(-g1, y, 1.), y, y);
+    w = __fma_rn(__fma_rn(-g1, g1, x), half_of(y1), g1);
+    iw = __fma_rn(__fma_rn(-w, y1, 1.), y1, y1);
+}
+
+/* Running extremes of the bit patterns that the steps above do not cover. */
+struct Odd {
+    uint32_t lo = 0, hi = 0, hn = 0xffffffffu;
+    __device__ __forceinline__ void divisor(double b)
+    {
+        lo = max(lo, (uint32_t)__double2loint(b));
+        const uint32_t h = (uint32_t)__double2hiint(b);
+        hi = max(hi, h);
+        hn = min(hn, h);
+    }
+    __device__ __forceinline__ void offset(double u) /* 0, or not below 2^-400 */
+    {
+        hn = min(hn, ((uint32_t)__double2hiint(u) & 0x7fffffffu) - 1u);
+    }
+    /* significand's low word 11..10 or 11..11, a divisor (positive) above 2^800 or not
+     * finite, below 2^-400 */
+    __device__ __forceinline__ bool any() const { return lo >= 0xfffffffeu || hi > 0x71f00000u || hn < 0x26f00000u; }
+};
+
+/* What the two radii of a pair share: the reference's sub-expressions in x, y and the halo's
+ * constants (record lt_rec64, the same roundings). */
+struct MdShared {
+    double xx, xxc, yyc, X1, Y1, Z1, Z2, yc, ycc, cxx;
+};
+__device__ __forceinline__ MdShared md_shared(const lt_rec64 &h, double x, double y)
+{
+    MdShared s;
+    s.xx = M(x, x);
+    s.xxc = quot(s.xx, h.cxro, h.cxro_inv);
+    s.yyc = quot(M(y, y), h.cyro, h.cyro_inv);
+    const double sx = M(h.sqe2, x);
+    s.X1 = quot(M(sx, x), h.cxro, h.cxro_inv);
+    s.Y1 = quot(M(M(sx, y), h.cx1), h.cyro, h.cyro_inv);
+    s.Z1 = quot(M(M(h.sqe2, y), y), h.cyro, h.cyro_inv);
+    s.Z2 = quot(M(h.k4, y), h.cyro, h.cyro_inv);
+    s.yc = M(y, h.cx1inv);
+    s.ycc = M(s.yc, h.cx1inv);
+    s.cxx = M(M(h.cx1sq, x), x);
+    return s;
+}
+__device__ __forceinline__ Mat mdci05(const lt_rec64 &h, const MdShared &s, double x, double y, double r2, double tsr,
+                                      Odd &odd)
+{
+    const double w2 = A(A(r2, s.xxc), s.yyc);
+    double w, iw;
+    sqrt_rn(w2, w, iw);
+    const double sw = M(h.sqe2, w);
+    const double d1 = S(sw, s.yc);
+    const double den1 = A(s.cxx, M(d1, d1));
+    const double num2 = S(tsr, y);
+    const double den2 = A(s.xx, M(num2, num2));
+    const double i1 = rcp_rn(den1), i2 = rcp_rn(den2);
+    const double n2 = quot(num2, den2, i2);
+    double t = A(S(quot(s.X1, w, iw), sw), s.yc);
+    const double didxre = M(h.ci, A(quot(M(h.cx1, t), den1, i1), n2));
+    t = S(quot(s.Y1, w, iw), x);
+    const double didyre = M(h.ci, A(quot(t, den1, i1), quot(x, den2, i2)));
+    t = S(S(M(sw, h.cx1inv), s.ycc), s.Z2);
+    t = A(t, M(quot(s.Z1, w, iw), h.cx1inv));
+    const double didyim = M(h.ci, S(quot(t, den1, i1), n2));
+    odd.divisor(w2);
+    odd.divisor(w);
+    odd.divisor(den1);
+    odd.divisor(den2);
+    Mat r;
+    r.a = M(h.b0, didxre);
+    r.b = r.d = M(h.b0, didyre);
+    r.c = M(h.b0, didyim);
+    return r;
+}
+
 /* two-step rotation back to the sky frame, src/gradient2.cpp:146-156 */
 __device__ __forceinline__ void rotate_acc(const Mat &h, double cs, double sn, Mat &acc)
 {
@@ -188,26 +296,28 @@ __device__ __forceinline__ void rotate_acc(const Mat &h, double cs, double sn, M
     acc.d = A(acc.d, A(M(sn, ma), M(cs, md)));
 }
 
-/* One halo's Hessian added to the run accumulator `acc`: dPIE src/gradient2.cpp:92-205;
- * PIEMD (one mdci05 term) and SIS restated with the same rounding discipline. */
+/* One halo's halo-frame Hessian by IEEE operations (dPIE src/gradient2.cpp:92-205, PIEMD = one
+ * mdci05 term): the pairs with an odd operand, out of line. */
 template <int TYPE>
-__device__ __forceinline__ void hess_pair(const lt_rec64 &h, double px, double py, Mat &acc)
+__device__ __noinline__ void hess_ieee(const lt_rec64 &h, double u, double v, Mat &m)
 {
-    const double tx = S(px, h.x0), ty = S(py, h.y0);
-    const double u = A(M(tx, h.cs), M(ty, h.sn));
-    const double v = S(M(ty, h.cs), M(tx, h.sn));
-    Mat m;
+    m = mdci05(u, v, h.eps, h.rc, h.b0);
     if (TYPE == 81) {
         const double t05 = V(h.rcut, S(h.rcut, h.rc));
-        Mat core = mdci05(u, v, h.eps, h.rc, h.b0);
         const Mat cut = mdci05(u, v, h.eps, h.rcut, h.b0);
-        m.a = M(t05, S(core.a, cut.a));
-        m.b = M(t05, S(core.b, cut.b));
-        m.c = M(t05, S(core.c, cut.c));
-        m.d = M(t05, S(core.d, cut.d));
-    } else if (TYPE == 8) {
-        m = mdci05(u, v, h.eps, h.rc, h.b0);
-    } else {
+        m.a = M(t05, S(m.a, cut.a));
+        m.b = M(t05, S(m.b, cut.b));
+        m.c = M(t05, S(m.c, cut.c));
+        m.d = M(t05, S(m.d, cut.d));
+    }
+}
+
+/* One halo's halo-frame Hessian at offset (u, v) with the reference's roundings; false where an
+ * operand is odd (hess_ieee then gives it).  SIS restated with the same rounding discipline. */
+template <int TYPE>
+__device__ __forceinline__ bool hess_frame(const lt_rec64 &h, double u, double v, Mat &m)
+{
+    if (TYPE == 5) {
         const double e = h.eps;
         const double q = A(M(M(u, u), S(1., e)), M(M(v, v), A(1., e)));
         const double r = R(q);
@@ -215,8 +325,48 @@ __device__ __forceinline__ void hess_pair(const lt_rec64 &h, double px, double p
         m.a = M(M(k, v), v);
         m.c = M(M(k, u), u);
         m.b = m.d = M(M(-k, u), v);
+        return true;
     }
-    rotate_acc(m, h.cs, h.sn, acc);
+    Odd odd;
+    odd.offset(u);
+    odd.offset(v);
+    const MdShared s = md_shared(h, u, v);
+    m = mdci05(h, s, u, v, h.rc2, h.tsr_c, odd);
+    if (TYPE == 81) {
+        const Mat cut = mdci05(h, s, u, v, h.rcut2, h.tsr_t, odd);
+        m.a = M(h.t05, S(m.a, cut.a));
+        m.b = m.d = M(h.t05, S(m.b, cut.b));
+        m.c = M(h.t05, S(m.c, cut.c));
+    }
+    return !odd.any();
+}
+
+/* One halo's Hessians at P pixels of a row added to the run accumulators.  220 FP64 operations
+ * a dPIE pair; the odd operands' branch is taken once in ~10^9 pairs. */
+template <int TYPE, int P>
+__device__ __forceinline__ void hess_pairs(const lt_rec64 &h, const double (&px)[P], double py, Mat (&acc)[P])
+{
+    const double ty = S(py, h.y0);
+    double u[P], v[P];
+    Mat m[P];
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < P; k++) {
+        const double tx = S(px[k], h.x0);
+        u[k] = A(M(tx, h.cs), M(ty, h.sn));
+        v[k] = S(M(ty, h.cs), M(tx, h.sn));
+        ok &= hess_frame<TYPE>(h, u[k], v[k], m[k]);
+    }
+    if (TYPE != 5 && !ok) {
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            Mat t;
+            hess_ieee<TYPE>(h, u[k], v[k], t);
+            m[k] = t;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < P; k++) rotate_acc(m[k], h.cs, h.sn, acc[k]);
 }
 } // namespace ex
 
