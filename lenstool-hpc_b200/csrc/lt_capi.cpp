@@ -268,7 +268,13 @@ lt_status lt_create(int device, size_t budget, lt_context **out)
     ctx->shape[LT_FP32C][OP_HESS | OP_POT] = LT_SHAPE4(2, 2, 256, 128);
     ctx->shape[LT_FP32C][OP_GRAD] = LT_SHAPE4(2, 2, 256, 128);
     cudaSetDevice(device);
-    if (configure_kernels32() != cudaSuccess) {
+    bool ok = configure_kernels32() == cudaSuccess && configure_tree64() == cudaSuccess;
+    if (ok) {
+        /* the device's first context (after a reset its module data is new) */
+        std::lock_guard<std::mutex> lock(g_ctx_mu);
+        if (device >= 64 || g_contexts[device] == 0) ok = tree_tables() == cudaSuccess;
+    }
+    if (!ok) {
         cudaGetLastError();
         delete ctx;
         return LT_ERR_CUDA;
@@ -382,7 +388,19 @@ lt_status lt_catalog_upload(lt_context *ctx, const lt_halo_soa *s, lt_catalog **
     cat->nhalos = s->nhalos;
     cat->host_recs.resize(s->nhalos);
     cat->host_types.assign(s->type, s->type + s->nhalos);
-    for (int i = 0; i < s->nhalos; i++) pack_one(s, i, cat->host_recs[i]);
+    double lo[2] = {0., 0.}, hi[2] = {0., 0.};
+    for (int i = 0; i < s->nhalos; i++) {
+        pack_one(s, i, cat->host_recs[i]);
+        const double e = s->ellipticity_potential[i], r = (1. + e) / (1. - e); /* 1/q; SIS: 1/q^2 */
+        cat->sum_iq += s->type[i] == 5 ? std::sqrt(r) : r;
+        cat->sum_iq2 += s->type[i] == 5 ? r : r * r;
+        const double p[2] = {s->position_x[i], s->position_y[i]};
+        for (int k = 0; k < 2; k++) {
+            lo[k] = i ? std::min(lo[k], p[k]) : p[k];
+            hi[k] = i ? std::max(hi[k], p[k]) : p[k];
+        }
+    }
+    cat->box = (hi[0] - lo[0]) * (hi[1] - lo[1]);
     std::vector<lt_chunk> ch = make_chunks(s->type, s->nhalos, LT_CHUNK);
     std::vector<double> w(s->nhalos);
     for (int i = 0; i < s->nhalos; i++) w[i] = cat->host_recs[i].w;
@@ -510,6 +528,7 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
     a.scale = scale;
     a.status = ctx->status;
     cudaStream_t s = (cudaStream_t)stream;
+    const int side = call_side(ctx, cat, op, precision, a);
     /* the kernels of one band of rows (the whole grid for device outputs) */
     auto launch = [&](GridArgs &b) -> int {
         if (cat->nhalos == 0) {
@@ -519,22 +538,7 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
             count_launch(1);
             return launch_epilogue_zero(b, ctx->num_sms, s);
         }
-        if (precision == LT_FP64 && (op & OP_HESS)) {
-            /* the Hessian with the reference's rounding sequence; with the potential (its
-             * own records and registers) as two launches, each writing its planes */
-            const int n = b.nout;
-            int pot = n;
-            if (op & OP_POT)
-                for (pot = 0; pot < n && b.kinds[pot] != KIND_POT;) pot++;
-            b.nout = pot;
-            int err = launch_grid64_tiled(OP_HEX, b, ctx->num_sms, s, ctx->shape[LT_FP64][op & 7]);
-            if (err != cudaSuccess || pot == n) return err;
-            b.nout = 1;
-            b.kinds[0] = KIND_POT;
-            b.out[0] = b.out[pot];
-            return launch_grid64_tiled(OP_POT, b, ctx->num_sms, s, ctx->shape[LT_FP64][OP_POT]);
-        }
-        if (precision != LT_FP32C) return launch_grid64_tiled(op, b, ctx->num_sms, s, ctx->shape[precision][op & 7]);
+        if (precision != LT_FP32C) return launch_fp64(ctx, cat, op, precision, b, side, s);
         return launch_fp32c(ctx, cat, op, b, s);
     };
     if (!host) {
@@ -545,12 +549,13 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
     /* Host outputs: the grid in bands of rows, each band's planes copied to the host on a
      * second stream while the next bands compute.  Every band is launched before the first
      * copy is issued, since a copy into pageable memory returns only once it is done.
-     * Bands start on multiples of 8 rows, the kernels' tile height, so every warp covers
-     * the pixels it covers in one launch over the whole grid and the maps are the same
-     * bit for bit. */
+     * Bands start on multiples of the kernels' tile height (8 rows, or the tile side of the
+     * interpolated sums), so every tile covers the pixels it covers in one launch over the
+     * whole grid and the maps are the same bit for bit. */
     int band = (int)(((long)g->ny + kHostBands - 1) / kHostBands);
-    band = (band + 7) / 8 * 8;
     if (band < kMinBandRows) band = kMinBandRows;
+    const int tile_rows = side ? side : 8;
+    band = (band + tile_rows - 1) / tile_rows * tile_rows;
     if (!ctx->copy_stream) {
         cudaError_t e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "copy stream");
@@ -582,6 +587,34 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
     if (err != cudaSuccess) return cuda_fail(ctx, (cudaError_t)err, "grid kernel launch or result copy");
     if (se != cudaSuccess) return cuda_fail(ctx, se, "result copy");
     return lt_synchronize(ctx, stream);
+}
+
+int lt::call_side(const lt_context *ctx, const lt_catalog *cat, int op, int precision, const GridArgs &a)
+{
+    if (precision == LT_FP32C || cat->nhalos == 0) return 0;
+    if (precision == LT_FP64 && (op & OP_HESS)) op &= ~OP_HESS; /* every pair, in the reference's order */
+    return op ? tree_side(cat, op, a.nx, a.ny, a.dx, a.dy, ctx->num_sms) : 0;
+}
+
+int lt::launch_fp64(lt_context *ctx, const lt_catalog *cat, int op, int precision, GridArgs &a, int side, void *stream)
+{
+    if (precision == LT_FP64 && (op & OP_HESS)) {
+        /* the Hessian with the reference's rounding sequence; with the potential (its own
+         * records and registers) as two launches, each writing its planes */
+        const int n = a.nout;
+        int pot = n;
+        if (op & OP_POT)
+            for (pot = 0; pot < n && a.kinds[pot] != KIND_POT;) pot++;
+        a.nout = pot;
+        const int err = launch_grid64_tiled(OP_HEX, a, ctx->num_sms, stream, ctx->shape[LT_FP64][op & 7]);
+        if (err != cudaSuccess || pot == n) return err;
+        a.nout = 1;
+        a.kinds[0] = KIND_POT;
+        a.out[0] = a.out[pot];
+        op = OP_POT;
+    }
+    if (side) return launch_tree64(cat, op, a, side, ctx->num_sms, stream);
+    return launch_grid64_tiled(op, a, ctx->num_sms, stream, ctx->shape[precision][op & 7]);
 }
 
 /* Tile bookkeeping shared by the launchers. */

@@ -438,7 +438,7 @@ int chi2_launch(lt_context *ctx, const lt_catalog *cat, Chi2Buf &b, bool sources
     } else if (precision == LT_FP32C) {
         err = launch_fp32c(ctx, cat, OP_GRAD, a, s);
     } else {
-        err = launch_grid64_tiled(OP_GRAD, a, ctx->num_sms, s, ctx->shape[precision][OP_GRAD]);
+        err = launch_fp64(ctx, cat, OP_GRAD, precision, a, call_side(ctx, cat, OP_GRAD, precision, a), s);
     }
     if (err != cudaSuccess) return err;
     (void)link;

@@ -41,6 +41,8 @@ struct lt_catalog {
     size_t bytes = 0;
     std::vector<lt_rec64> host_recs;     /* packed records, host copy */
     std::vector<int32_t> host_types;     /* profile type per halo */
+    double sum_iq = 0, sum_iq2 = 0, box = 0; /* sums of 1/q and 1/q^2 over the halos, area of their
+                                            bounding box, at upload (tree_side's estimate) */
     void *aux = nullptr;                 /* FP32C records and chunks, device */
     size_t aux_bytes = 0;
     void *stage = nullptr;               /* device staging of host parameters (lt_catalog_update) */
@@ -101,6 +103,15 @@ std::vector<lt_chunk> make_chunks(const int32_t *type, int n, int max_chunk, con
 
 lt_status run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g, int precision, int op, int kmap, double D,
                    double mult, double scale, int nout, const int *kinds, double *const *outs, void *stream);
+/* far halos interpolated over tiles (lt_tree64.cu) */
+int tree_tables();
+int configure_tree64();
+int tree_side(const lt_catalog *cat, int op, int nx, int ny, double dx, double dy, int num_sms);
+int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side, int num_sms, void *stream);
+/* FP64 sums `op` of one precision on a grid or a band of one; `side`: tree_side of the whole grid */
+int launch_fp64(lt_context *ctx, const lt_catalog *cat, int op, int precision, GridArgs &a, int side, void *stream);
+/* the tile side of a call's closed-form sums (0: direct) */
+int call_side(const lt_context *ctx, const lt_catalog *cat, int op, int precision, const GridArgs &a);
 int launch_grid64_tiled(int op, GridArgs &a, int num_sms, void *stream, int shape);
 int launch_epilogue_zero(const GridArgs &a, int num_sms, void *stream);
 int launch_grid64_list(int op, GridArgs &a, int num_sms, void *stream);
