@@ -167,7 +167,30 @@ __device__ __forceinline__ void close64(Acc64<OP, P> &acc, int k, double &d)
  * further: this replaces a per-term compensated (Kahan) update at a quarter of its cost. */
 constexpr int kBlock32 = 8;
 
-/* Sums of one pixel.  FP64: convergence, shear and potential (halo-frame Hessians are
+/* The FP32 sums of a thread's P pixels; two pixels packed (f2). */
+template <int P>
+struct Lanes {
+    float a[P];
+    __device__ __forceinline__ void zero()
+    {
+#pragma unroll
+        for (int k = 0; k < P; k++) a[k] = 0.f;
+    }
+    __device__ __forceinline__ float get(int k) const { return a[k]; }
+    __device__ __forceinline__ void set(int k, float x) { a[k] = x; }
+};
+template <>
+struct Lanes<2> {
+    f2 a;
+    __device__ __forceinline__ void zero() { a.v = 0ull; }
+    __device__ __forceinline__ float get(int k) const { return k ? p2::hi(a) : p2::lo(a); }
+    __device__ __forceinline__ void set(int k, float x)
+    {
+        a = k ? p2::pack(p2::lo(a), x) : p2::pack(x, p2::hi(a));
+    }
+};
+
+/* Sums of P pixels.  FP64: convergence, shear and potential (halo-frame Hessians are
  * rotated to the sky frame before they are added) and the deflection.  FP32: the running
  * block sums, and the magnitudes of the FP32 terms from which the error of the FP32 part
  * is estimated (fp32c_total): sum kappa_i^2 and sum (|gamma1_i| + |gamma2_i|)^2 (halo
@@ -175,17 +198,24 @@ constexpr int kBlock32 = 8;
 template <int P>
 struct Acc32 {
     double kap[P], g1[P], g2[P], psi[P], gx[P], gy[P];
-    float bk[P], bg1[P], bg2[P], bp[P], bgx[P], bgy[P];
-    float mk[P], mg[P], ml[P];
+    Lanes<P> bk, bg1, bg2, bp, bgx, bgy;
+    Lanes<P> mk, mg, ml;
 };
 
-/* Zero the sums of pixel k. */
 template <int P>
-__device__ __forceinline__ void acc32_zero(Acc32<P> &acc, int k)
+__device__ __forceinline__ void acc32_zero(Acc32<P> &acc)
 {
-    acc.kap[k] = acc.g1[k] = acc.g2[k] = acc.psi[k] = acc.gx[k] = acc.gy[k] = 0.;
-    acc.bk[k] = acc.bg1[k] = acc.bg2[k] = acc.bp[k] = acc.bgx[k] = acc.bgy[k] = 0.f;
-    acc.mk[k] = acc.mg[k] = acc.ml[k] = 0.f;
+#pragma unroll
+    for (int k = 0; k < P; k++) acc.kap[k] = acc.g1[k] = acc.g2[k] = acc.psi[k] = acc.gx[k] = acc.gy[k] = 0.;
+    acc.bk.zero();
+    acc.bg1.zero();
+    acc.bg2.zero();
+    acc.bp.zero();
+    acc.bgx.zero();
+    acc.bgy.zero();
+    acc.mk.zero();
+    acc.mg.zero();
+    acc.ml.zero();
 }
 
 /* Join the FP32 block sums to the FP64 sums, with the chunk's Kmap weight w (1 outside
@@ -196,21 +226,26 @@ __device__ __forceinline__ void fold32(Acc32<P> &acc, double w)
 #pragma unroll
     for (int k = 0; k < P; k++) {
         if (OP & OP_HESS) {
-            acc.kap[k] = __fma_rn(w, (double)acc.bk[k], acc.kap[k]);
-            acc.g1[k] = __fma_rn(w, (double)acc.bg1[k], acc.g1[k]);
-            acc.g2[k] = __fma_rn(w, (double)acc.bg2[k], acc.g2[k]);
-            acc.ml[k] = __fmaf_rn((float)w, acc.bk[k], acc.ml[k]);
-            acc.bk[k] = acc.bg1[k] = acc.bg2[k] = 0.f;
+            acc.kap[k] = __fma_rn(w, (double)acc.bk.get(k), acc.kap[k]);
+            acc.g1[k] = __fma_rn(w, (double)acc.bg1.get(k), acc.g1[k]);
+            acc.g2[k] = __fma_rn(w, (double)acc.bg2.get(k), acc.g2[k]);
+            acc.ml.set(k, __fmaf_rn((float)w, acc.bk.get(k), acc.ml.get(k)));
         }
-        if (OP & OP_POT) {
-            acc.psi[k] = __dadd_rn(acc.psi[k], (double)acc.bp[k]);
-            acc.bp[k] = 0.f;
-        }
+        if (OP & OP_POT) acc.psi[k] = __dadd_rn(acc.psi[k], (double)acc.bp.get(k));
         if (OP & OP_GRAD) {
-            acc.gx[k] = __dadd_rn(acc.gx[k], (double)acc.bgx[k]);
-            acc.gy[k] = __dadd_rn(acc.gy[k], (double)acc.bgy[k]);
-            acc.bgx[k] = acc.bgy[k] = 0.f;
+            acc.gx[k] = __dadd_rn(acc.gx[k], (double)acc.bgx.get(k));
+            acc.gy[k] = __dadd_rn(acc.gy[k], (double)acc.bgy.get(k));
         }
+    }
+    if (OP & OP_HESS) {
+        acc.bk.zero();
+        acc.bg1.zero();
+        acc.bg2.zero();
+    }
+    if (OP & OP_POT) acc.bp.zero();
+    if (OP & OP_GRAD) {
+        acc.bgx.zero();
+        acc.bgy.zero();
     }
 }
 
@@ -294,6 +329,61 @@ __device__ __forceinline__ void eval64_chunk(const lt_rec64 *recs, const lt_nie6
     }
 }
 
+/* The FP32 terms of one record at a thread's pixels (halo-frame offsets u, v) added to the
+ * block sums. */
+template <int OP, int P, int TYPE>
+__device__ __forceinline__ void terms32(const lt_rec32 &r, const float (&u)[P], const float (&v)[P], Acc32<P> &acc)
+{
+#pragma unroll
+    for (int k = 0; k < P; k++) {
+        const Nie32 n = nie32<TYPE>(r, u[k], v[k]);
+        if (OP & OP_HESS) {
+            const KG32 t = hess32<TYPE>(r, u[k], v[k], n);
+            acc.bk.set(k, __fadd_rn(acc.bk.get(k), t.k));
+            acc.bg1.set(k, __fmaf_rn(t.g1, r.c2t, __fmaf_rn(-t.g2, r.s2t, acc.bg1.get(k))));
+            acc.bg2.set(k, __fmaf_rn(t.g1, r.s2t, __fmaf_rn(t.g2, r.c2t, acc.bg2.get(k))));
+            const float ag = __fadd_rn(fabsf(t.g1), fabsf(t.g2));
+            acc.mk.set(k, __fmaf_rn(t.k, t.k, acc.mk.get(k)));
+            acc.mg.set(k, __fmaf_rn(ag, ag, acc.mg.get(k)));
+        }
+        if (OP & (OP_GRAD | OP_POT)) {
+            const G32 t = grad32<TYPE>(r, u[k], v[k], n);
+            if (OP & OP_GRAD) {
+                acc.bgx.set(k, __fmaf_rn(t.x, r.cs, __fmaf_rn(-t.y, r.sn, acc.bgx.get(k))));
+                acc.bgy.set(k, __fmaf_rn(t.y, r.cs, __fmaf_rn(t.x, r.sn, acc.bgy.get(k))));
+            }
+            if (OP & OP_POT) acc.bp.set(k, __fadd_rn(acc.bp.get(k), pot32<TYPE>(r, u[k], v[k], n, t)));
+        }
+    }
+}
+
+/* terms32 of a cut dPIE at two pixels, packed: the same operations and roundings. */
+template <int OP>
+__device__ __forceinline__ void terms32x2(const lt_rec32 &r, f2 u, f2 v, Acc32<2> &acc)
+{
+    using namespace p2;
+    const Nie2 n = nie32x2(r, u, v);
+    if (OP & OP_HESS) {
+        const KG2 t = hess32x2(r, u, v, n);
+        const f2 c2 = dup(r.c2t), s2 = dup(r.s2t);
+        acc.bk.a = add(acc.bk.a, t.k);
+        acc.bg1.a = fma(t.g1, c2, fma(t.g2, dup(-r.s2t), acc.bg1.a));
+        acc.bg2.a = fma(t.g1, s2, fma(t.g2, c2, acc.bg2.a));
+        const f2 ag = pack(__fadd_rn(fabsf(lo(t.g1)), fabsf(lo(t.g2))), __fadd_rn(fabsf(hi(t.g1)), fabsf(hi(t.g2))));
+        acc.mk.a = fma(t.k, t.k, acc.mk.a);
+        acc.mg.a = fma(ag, ag, acc.mg.a);
+    }
+    if (OP & (OP_GRAD | OP_POT)) {
+        const G2 t = grad32x2(r, u, v, n);
+        if (OP & OP_GRAD) {
+            const f2 cs = dup(r.cs);
+            acc.bgx.a = fma(t.x, cs, fma(t.y, dup(-r.sn), acc.bgx.a));
+            acc.bgy.a = fma(t.y, cs, fma(t.x, dup(r.sn), acc.bgy.a));
+        }
+        if (OP & OP_POT) acc.bp.a = add(acc.bp.a, pot32x2(r, u, v, n, t));
+    }
+}
+
 /* One chunk of FP32 records (at most 128) for the pixels px[0..P) of row py, the lane's
  * pixels (ix .. ix + P - 1, iy) of grid `a`.  Every record of an FP32C chunk has the same
  * Kmap weight. */
@@ -312,13 +402,24 @@ __device__ __forceinline__ void eval32_chunk(const lt_rec32 *recs, const lt_rec6
 #pragma unroll 1
         for (int h = h0; h < h0 + n; h++) {
             const lt_rec32 &r = recs[h];
+            constexpr bool packed = P == 2 && TYPE == 81;
             float u[P], v[P];
+            f2 u2, v2;
             const float ty = __double2float_rn(__dsub_rn(py, r.y0));
+            if constexpr (packed) {
+                using namespace p2;
+                const f2 t = pack(__double2float_rn(__dsub_rn(px[0], r.x0)), __double2float_rn(__dsub_rn(px[1], r.x0)));
+                u2 = fma(t, dup(r.cs), dup(__fmul_rn(ty, r.sn)));
+                /* ty cs - (tx sn), the product rounded first */
+                v2 = fma(dup(ty), dup(r.cs), mul(t, dup(-r.sn)));
+                u[0] = lo(u2), u[1] = hi(u2), v[0] = lo(v2), v[1] = hi(v2);
+            } else {
 #pragma unroll
-            for (int k = 0; k < P; k++) {
-                const float tx = __double2float_rn(__dsub_rn(px[k], r.x0));
-                u[k] = __fmaf_rn(tx, r.cs, __fmul_rn(ty, r.sn));
-                v[k] = __fmaf_rn(ty, r.cs, -__fmul_rn(tx, r.sn));
+                for (int k = 0; k < P; k++) {
+                    const float tx = __double2float_rn(__dsub_rn(px[k], r.x0));
+                    u[k] = __fmaf_rn(tx, r.cs, __fmul_rn(ty, r.sn));
+                    v[k] = __fmaf_rn(ty, r.cs, -__fmul_rn(tx, r.sn));
+                }
             }
             bool near = false;
             if ((mask >> (h - h0)) & 1ull) {
@@ -341,28 +442,10 @@ __device__ __forceinline__ void eval32_chunk(const lt_rec32 *recs, const lt_rec6
                     }
                     if (OP & OP_POT) acc.psi[k] = __dadd_rn(acc.psi[k], pot_term<TYPE>(rn, px[k], py));
                 }
+            } else if constexpr (packed) {
+                terms32x2<OP>(r, u2, v2, acc);
             } else {
-#pragma unroll
-                for (int k = 0; k < P; k++) {
-                    const Nie32 n = nie32<TYPE>(r, u[k], v[k]);
-                    if (OP & OP_HESS) {
-                        const KG32 t = hess32<TYPE>(r, u[k], v[k], n);
-                        acc.bk[k] = __fadd_rn(acc.bk[k], t.k);
-                        acc.bg1[k] = __fmaf_rn(t.g1, r.c2t, __fmaf_rn(-t.g2, r.s2t, acc.bg1[k]));
-                        acc.bg2[k] = __fmaf_rn(t.g1, r.s2t, __fmaf_rn(t.g2, r.c2t, acc.bg2[k]));
-                        const float ag = __fadd_rn(fabsf(t.g1), fabsf(t.g2));
-                        acc.mk[k] = __fmaf_rn(t.k, t.k, acc.mk[k]);
-                        acc.mg[k] = __fmaf_rn(ag, ag, acc.mg[k]);
-                    }
-                    if (OP & (OP_GRAD | OP_POT)) {
-                        const G32 t = grad32<TYPE>(r, u[k], v[k], n);
-                        if (OP & OP_GRAD) {
-                            acc.bgx[k] = __fmaf_rn(t.x, r.cs, __fmaf_rn(-t.y, r.sn, acc.bgx[k]));
-                            acc.bgy[k] = __fmaf_rn(t.y, r.cs, __fmaf_rn(t.x, r.sn, acc.bgy[k]));
-                        }
-                        if (OP & OP_POT) acc.bp[k] = __fadd_rn(acc.bp[k], pot32<TYPE>(r, u[k], v[k], n, t));
-                    }
-                }
+                terms32<OP, P, TYPE>(r, u, v, acc);
             }
             if ((h & (kBlock32 - 1)) == kBlock32 - 1) fold32<OP, P>(acc, wchunk);
         }
@@ -406,8 +489,8 @@ __device__ __forceinline__ void fp32c_total(const Acc32<P> &acc, int k, double D
     psi = acc.psi[k];
     const double omk = sub(1., mul(kap, D)), g1d = mul(g1, D), g2d = mul(g2, D);
     det = sub(sub(mul(omk, omk), mul(g1d, g1d)), mul(g2d, g2d));
-    const float dk = __fmaf_rn(kEpsTerm32 * kSpread32, __fsqrt_rn(acc.mk[k]), __fmul_rn(kEpsBlock32, acc.ml[k]));
-    const float dg = __fmul_rn(kEpsTerm32 * kSpread32, __fsqrt_rn(acc.mg[k]));
+    const float dk = __fmaf_rn(kEpsTerm32 * kSpread32, __fsqrt_rn(acc.mk.get(k)), __fmul_rn(kEpsBlock32, acc.ml.get(k)));
+    const float dg = __fmul_rn(kEpsTerm32 * kSpread32, __fsqrt_rn(acc.mg.get(k)));
     const double gd = sqr(add(mul(g1d, g1d), mul(g2d, g2d)));
     det_err = mul(mul(2., D), add(mul(fabs(omk), (double)dk), mul(gd, (double)dg)));
 }

@@ -199,10 +199,8 @@ __global__ void __launch_bounds__(NT, MINB) grid32c_kernel(const C32Args A)
             iy = ty * kTileH + oy;
             py = pixel_y(a, iy < a.ny ? iy : a.ny - 1);
 #pragma unroll
-            for (int k = 0; k < P; k++) {
-                px[k] = pixel_x(a, (ix + k) < a.nx ? ix + k : a.nx - 1);
-                acc32_zero(acc, k);
-            }
+            for (int k = 0; k < P; k++) px[k] = pixel_x(a, (ix + k) < a.nx ? ix + k : a.nx - 1);
+            acc32_zero(acc);
         }
         if (tid == 0 && s + 1 < steps) issue(s + 1);
         const int b = (int)(s & 1);

@@ -202,10 +202,8 @@ __device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_
     double px[P];
     Acc32<P> acc;
 #pragma unroll
-    for (int k = 0; k < P; k++) {
-        px[k] = pixel_x(a, (ix + k) < a.nx ? ix + k : a.nx - 1);
-        acc32_zero(acc, k);
-    }
+    for (int k = 0; k < P; k++) px[k] = pixel_x(a, (ix + k) < a.nx ? ix + k : a.nx - 1);
+    acc32_zero(acc);
     bool ok = walk_chunks(st, it.chunks32, it.nchunks32, a.recs, it.recs32, status,
                           [&](const lt_chunk &c, const unsigned char *buf) {
                               if (c.pad & CHUNK_FP32) {
