@@ -71,11 +71,22 @@ lt_status lt::cuda_fail(lt_context *ctx, cudaError_t e, const char *what)
 
 lt_status lt::dev_alloc(lt_context *ctx, void **p, size_t bytes)
 {
-    if (ctx->used + bytes > ctx->budget) {
+    auto give_back = [&] { /* the kept workspace, if no call is in it */
+        if (!ctx->scratch || ctx->scratch_busy) return false;
+        dev_free(ctx, ctx->scratch, ctx->scratch_bytes);
+        ctx->scratch = nullptr;
+        ctx->scratch_bytes = 0;
+        return true;
+    };
+    if (ctx->used + bytes > ctx->budget && !(give_back() && ctx->used + bytes <= ctx->budget)) {
         set_error(ctx, "HBM budget exceeded: %zu in use + %zu requested > %zu", ctx->used, bytes, ctx->budget);
         return LT_ERR_BUDGET;
     }
     cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
+    if (e == cudaErrorMemoryAllocation && give_back()) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes ? bytes : 16);
+    }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
     ctx->used += bytes;
     return LT_OK;
@@ -88,20 +99,16 @@ void lt::dev_free(lt_context *ctx, void *p, size_t bytes)
     ctx->used -= bytes;
 }
 
-/* Device staging planes for host-pointer outputs, grown on demand. */
-lt_status lt::scratch_planes(lt_context *ctx, int n, size_t plane_bytes, double **planes)
+/* The kept workspace, grown on demand to `bytes`. */
+lt_status lt::scratch_alloc(lt_context *ctx, size_t bytes)
 {
-    size_t need = (size_t)n * plane_bytes;
-    if (need > ctx->scratch_bytes) {
-        dev_free(ctx, ctx->scratch, ctx->scratch_bytes);
-        ctx->scratch = nullptr;
-        ctx->scratch_bytes = 0;
-        lt_status st = dev_alloc(ctx, &ctx->scratch, need);
-        if (st != LT_OK) return st;
-        ctx->scratch_bytes = need;
-    }
-    for (int i = 0; i < n; i++) planes[i] = (double *)((char *)ctx->scratch + (size_t)i * plane_bytes);
-    return LT_OK;
+    if (bytes <= ctx->scratch_bytes) return LT_OK;
+    dev_free(ctx, ctx->scratch, ctx->scratch_bytes);
+    ctx->scratch = nullptr;
+    ctx->scratch_bytes = 0;
+    lt_status st = dev_alloc(ctx, &ctx->scratch, bytes);
+    if (st == LT_OK) ctx->scratch_bytes = bytes;
+    return st;
 }
 
 /* Pixel list (and its counter, in the first 16 bytes) of the recomputation pass. */
@@ -494,10 +501,12 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
     const size_t plane = npix * sizeof(double);
     bool host = false;
     for (int i = 0; i < nout; i++) host |= !is_device_pointer(outs[i]);
+    const ScratchUse use(ctx, host);
     double *dev_out[LT_MAX_MAPS];
     if (host) {
-        lt_status st = scratch_planes(ctx, nout, plane, dev_out);
+        lt_status st = scratch_alloc(ctx, nout * plane);
         if (st != LT_OK) return st;
+        for (int i = 0; i < nout; i++) dev_out[i] = (double *)((char *)ctx->scratch + (size_t)i * plane);
     } else {
         for (int i = 0; i < nout; i++) dev_out[i] = outs[i];
     }

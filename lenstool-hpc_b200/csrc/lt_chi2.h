@@ -23,21 +23,20 @@ struct Chi2Dev {
     int n;
     double xmin, ymin, dx, dy;
     const double *ax, *ay;              /* deflection grid, n x n */
-    /* work */
+    /* work and results: one block of each per model, model m's at m x its size */
     double *bx, *by;                    /* source per system */
     int32_t *hits, *keys;               /* hit count and hit keys (2 * cell + lower) per system */
-    /* results */
     double *chi_terms;                  /* per observed image: its chi2 term */
-    double *chi2;                       /* [0]: chi2; written by the reduction */
-    int32_t *found;                     /* [0]: predicted images; [1]: 1 if a source overflowed */
+    double *chi2;                       /* one word a model */
+    int32_t *found;                     /* two words a model: predicted images; 1 if a source overflowed */
     int32_t *nfound;                    /* predicted images per system (<= LT_MAX_IMAGES) */
     double *fx, *fy;                    /* predicted images, nsys x LT_MAX_IMAGES */
 };
 
-/* Bytes of one evaluation's device buffers (systems, work, results, the n x n deflection
- * planes); with `mem`, also lays them out there and fills `c` (grid from the frame:
+/* Bytes of the device buffers of `nmodels` evaluations (systems, work and results of each
+ * model, the n x n deflection planes, which the models take in turn); with `mem`, also lays them out there and fills `c` (grid from the frame:
  * dx = (xmax - xmin)/(n - 1), src/chi_CPU_barycenter.cpp:104-105). */
-size_t chi2_layout(int nsys, int nimages, const lt_frame *f, int n, char *mem, Chi2Dev &c);
+size_t chi2_layout(int nsys, int nimages, const lt_frame *f, int n, char *mem, Chi2Dev &c, int nmodels = 1);
 
 /* Copy the systems (host arrays; `first` = index of each system's first image) into the
  * layout, stream-ordered; the host arrays must stay valid until the copies have run. */

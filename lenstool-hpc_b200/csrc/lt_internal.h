@@ -18,8 +18,12 @@ struct lt_context {
     size_t budget = 0, used = 0;
     std::mutex mu;
     std::string last_error;
+    /* workspace of the calls that return when their work is done (host-output planes, chi2),
+     * kept from call to call; dev_alloc gives it back when the budget or the device runs out and
+     * no call is in it (scratch_busy) */
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
+    bool scratch_busy = false;
     int32_t *status = nullptr; /* device status word written by kernels */
     void *ext = nullptr;       /* state of the batch and serving extensions */
     void *list = nullptr;      /* pixel list of the FP32C recomputation pass (+ count) */
@@ -97,7 +101,13 @@ void set_error(lt_context *ctx, const char *fmt, ...);
 lt_status cuda_fail(lt_context *ctx, cudaError_t e, const char *what);
 lt_status dev_alloc(lt_context *ctx, void **p, size_t bytes);
 void dev_free(lt_context *ctx, void *p, size_t bytes);
-lt_status scratch_planes(lt_context *ctx, int n, size_t plane_bytes, double **planes);
+lt_status scratch_alloc(lt_context *ctx, size_t bytes);
+/* marks the workspace in use for the rest of the caller's scope (which holds ctx->mu) */
+struct ScratchUse {
+    lt_context *ctx;
+    explicit ScratchUse(lt_context *c, bool use = true) : ctx(c) { ctx->scratch_busy = use; }
+    ~ScratchUse() { ctx->scratch_busy = false; }
+};
 bool is_device_pointer(const void *p);
 std::vector<lt_chunk> make_chunks(const int32_t *type, int n, int max_chunk, const double *dlsds = nullptr);
 
