@@ -270,10 +270,10 @@ lt_status lt_create(int device, size_t budget, lt_context **out)
         for (int o : {(int)OP_GRAD, (int)OP_HESS, (int)OP_POT, OP_HESS | OP_POT}) ctx->shape[p][o] = LT_SHAPE(2, 2);
     /* the reference-order Hessian: 1024^2 x 1000 halos 15.6 ms (2, 2: 16.2), 600^2 1.7 (2.0) */
     ctx->shape[LT_FP64][OP_HESS] = ctx->shape[LT_FP64][OP_HESS | OP_POT] = LT_SHAPE(1, 2);
-    ctx->shape[LT_FP32C][OP_HESS] = LT_SHAPE4(2, 2, 256, 128);
-    ctx->shape[LT_FP32C][OP_POT] = LT_SHAPE4(2, 2, 256, 128);
+    ctx->shape[LT_FP32C][OP_HESS] = LT_SHAPE4(2, 4, 128, 64);
+    ctx->shape[LT_FP32C][OP_POT] = LT_SHAPE4(2, 4, 128, 64);
     ctx->shape[LT_FP32C][OP_HESS | OP_POT] = LT_SHAPE4(2, 2, 256, 128);
-    ctx->shape[LT_FP32C][OP_GRAD] = LT_SHAPE4(2, 2, 256, 128);
+    ctx->shape[LT_FP32C][OP_GRAD] = LT_SHAPE4(2, 4, 128, 64);
     cudaSetDevice(device);
     bool ok = configure_kernels32() == cudaSuccess && configure_tree64() == cudaSuccess;
     if (ok) {

@@ -23,39 +23,44 @@ struct Acc64 {
 };
 
 /* One staged chunk: lt_rec64 records for OP_HEX, lt_nie64 otherwise (then acc.hxx, hyy and hxy
- * hold the convergence and shear sums until close64). */
-template <int OP, int P, int TYPE>
+ * hold the convergence and shear sums until close64).  U records of OP_HEX at a time. */
+template <int OP, int P, int TYPE, int U>
 __device__ __forceinline__ void eval_chunk64(const void *staged, int count, const double (&px)[P], double py,
                                              int kmap, Acc64<OP, P> &acc)
 {
+    if (OP & OP_HEX) {
+        const lt_rec64 *r = static_cast<const lt_rec64 *>(staged);
+        int h = 0;
+#pragma unroll 1
+        for (; h + U <= count; h += U) ex::hess_pairs<TYPE, P, U>(r + h, px, py, acc.run);
+        if (U > 1)
+#pragma unroll 1
+            for (; h < count; h++) ex::hess_pairs<TYPE, P, 1>(r + h, px, py, acc.run);
+        return;
+    }
 #pragma unroll 1
     for (int h = 0; h < count; h++) {
-        if (OP & OP_HEX) {
-            const lt_rec64 &r = static_cast<const lt_rec64 *>(staged)[h];
-            ex::hess_pairs<TYPE, P>(r, px, py, acc.run);
-        } else {
-            const lt_nie64 &r = static_cast<const lt_nie64 *>(staged)[h];
-            const double w = kmap ? r.w : 1.0;
+        const lt_nie64 &r = static_cast<const lt_nie64 *>(staged)[h];
+        const double w = kmap ? r.w : 1.0;
 #pragma unroll
-            for (int k = 0; k < P; k++) {
-                const Nie64 n = nie64<TYPE>(r, px[k], py);
-                if (OP & OP_GRAD) grad_nie<TYPE>(r, n, acc.gx[k], acc.gy[k]);
-                if (OP & OP_HESS) kg_nie<TYPE>(r, n, w, acc.hxx[k], acc.hyy[k], acc.hxy[k]);
-                if (OP & OP_POT) pot_nie<TYPE>(r, n, acc.psi[k]);
-            }
+        for (int k = 0; k < P; k++) {
+            const Nie64 n = nie64<TYPE>(r, px[k], py);
+            if (OP & OP_GRAD) grad_nie<TYPE>(r, n, acc.gx[k], acc.gy[k]);
+            if (OP & OP_HESS) kg_nie<TYPE>(r, n, w, acc.hxx[k], acc.hyy[k], acc.hxy[k]);
+            if (OP & OP_POT) pot_nie<TYPE>(r, n, acc.psi[k]);
         }
     }
 }
 
 /* eval_chunk64 over one staged chunk of any profile type. */
-template <int OP, int P>
+template <int OP, int P, int U = 1>
 __device__ __forceinline__ void eval_any64(const lt_chunk &c, const void *staged, const double (&px)[P], double py,
                                            int kmap, Acc64<OP, P> &acc)
 {
     switch (c.type) {
-    case 81: eval_chunk64<OP, P, 81>(staged, c.count, px, py, kmap, acc); break;
-    case 8: eval_chunk64<OP, P, 8>(staged, c.count, px, py, kmap, acc); break;
-    case 5: eval_chunk64<OP, P, 5>(staged, c.count, px, py, kmap, acc); break;
+    case 81: eval_chunk64<OP, P, 81, U>(staged, c.count, px, py, kmap, acc); break;
+    case 8: eval_chunk64<OP, P, 8, U>(staged, c.count, px, py, kmap, acc); break;
+    case 5: eval_chunk64<OP, P, 5, U>(staged, c.count, px, py, kmap, acc); break;
     default: break;
     }
 }
@@ -73,12 +78,12 @@ __device__ __forceinline__ const void *recs_of(const GridArgs &a, int start)
  * weight for a Kmap).  The Q pixels' dependent chains are independent of one another, so
  * the compiler interleaves them; nie_kg64's pinned rounding keeps each pair's value the
  * same for any Q and in every kernel. */
-template <int Q, int TYPE>
+template <int Q, int TYPE, int U>
 __device__ __forceinline__ void eval_nie_q(const lt_nie64 *recs, int count, const double (&px)[Q],
                                            const double (&py)[Q], int kmap, double (&kap)[Q], double (&g1)[Q],
                                            double (&g2)[Q])
 {
-#pragma unroll 1
+#pragma unroll U
     for (int h = 0; h < count; h++) {
         const lt_nie64 &r = recs[h];
 #pragma unroll
@@ -98,15 +103,15 @@ __device__ __forceinline__ void eval_nie_q(const lt_nie64 *recs, int count, cons
 }
 
 /* eval_nie_q over one staged chunk of any profile type. */
-template <int Q>
+template <int Q, int U = 1>
 __device__ __forceinline__ void eval_nie_chunk(const lt_chunk &c, const lt_nie64 *recs, const double (&px)[Q],
                                                const double (&py)[Q], int kmap, double (&kap)[Q], double (&g1)[Q],
                                                double (&g2)[Q])
 {
     switch (c.type) {
-    case 81: eval_nie_q<Q, 81>(recs, c.count, px, py, kmap, kap, g1, g2); break;
-    case 8: eval_nie_q<Q, 8>(recs, c.count, px, py, kmap, kap, g1, g2); break;
-    case 5: eval_nie_q<Q, 5>(recs, c.count, px, py, kmap, kap, g1, g2); break;
+    case 81: eval_nie_q<Q, 81, U>(recs, c.count, px, py, kmap, kap, g1, g2); break;
+    case 8: eval_nie_q<Q, 8, U>(recs, c.count, px, py, kmap, kap, g1, g2); break;
+    case 5: eval_nie_q<Q, 5, U>(recs, c.count, px, py, kmap, kap, g1, g2); break;
     default: break;
     }
 }
@@ -357,14 +362,29 @@ __device__ __forceinline__ void terms32(const lt_rec32 &r, const float (&u)[P], 
     }
 }
 
-/* terms32 of a cut dPIE at two pixels, packed: the same operations and roundings. */
+/* terms32 of a cut dPIE at two pixels, packed: the same operations and roundings, the terms and
+ * their addition to the block sums apart. */
+struct Terms2 {
+    KG2 h;
+    G2 g;
+    f2 p;
+};
+template <int OP, bool SKIP>
+__device__ __forceinline__ Terms2 terms32x2(const lt_rec32 &r, f2 u, f2 v)
+{
+    Terms2 t;
+    const Nie2 n = nie32x2(r, u, v);
+    if (OP & OP_HESS) t.h = hess32x2(r, u, v, n);
+    if (OP & (OP_GRAD | OP_POT)) t.g = grad32x2<SKIP>(r, u, v, n);
+    if (OP & OP_POT) t.p = pot32x2<SKIP>(r, u, v, n, t.g);
+    return t;
+}
 template <int OP>
-__device__ __forceinline__ void terms32x2(const lt_rec32 &r, f2 u, f2 v, Acc32<2> &acc)
+__device__ __forceinline__ void add32x2(const lt_rec32 &r, const Terms2 &s, Acc32<2> &acc)
 {
     using namespace p2;
-    const Nie2 n = nie32x2(r, u, v);
     if (OP & OP_HESS) {
-        const KG2 t = hess32x2(r, u, v, n);
+        const KG2 &t = s.h;
         const f2 c2 = dup(r.c2t), s2 = dup(r.s2t);
         acc.bk.a = add(acc.bk.a, t.k);
         acc.bg1.a = fma(t.g1, c2, fma(t.g2, dup(-r.s2t), acc.bg1.a));
@@ -373,21 +393,79 @@ __device__ __forceinline__ void terms32x2(const lt_rec32 &r, f2 u, f2 v, Acc32<2
         acc.mk.a = fma(t.k, t.k, acc.mk.a);
         acc.mg.a = fma(ag, ag, acc.mg.a);
     }
-    if (OP & (OP_GRAD | OP_POT)) {
-        const G2 t = grad32x2(r, u, v, n);
-        if (OP & OP_GRAD) {
-            const f2 cs = dup(r.cs);
-            acc.bgx.a = fma(t.x, cs, fma(t.y, dup(-r.sn), acc.bgx.a));
-            acc.bgy.a = fma(t.y, cs, fma(t.x, dup(r.sn), acc.bgy.a));
+    if (OP & OP_GRAD) {
+        const f2 cs = dup(r.cs);
+        acc.bgx.a = fma(s.g.x, cs, fma(s.g.y, dup(-r.sn), acc.bgx.a));
+        acc.bgy.a = fma(s.g.y, cs, fma(s.g.x, dup(r.sn), acc.bgy.a));
+    }
+    if (OP & OP_POT) acc.bp.a = add(acc.bp.a, s.p);
+}
+
+/* Halo-frame offsets of a thread's two pixels from a record's centre. */
+__device__ __forceinline__ void frame32x2(const lt_rec32 &r, const double (&px)[2], double py, f2 &u, f2 &v)
+{
+    using namespace p2;
+    const float ty = __double2float_rn(__dsub_rn(py, r.y0));
+    const f2 t = pack(__double2float_rn(__dsub_rn(px[0], r.x0)), __double2float_rn(__dsub_rn(px[1], r.x0)));
+    u = fma(t, dup(r.cs), dup(__fmul_rn(ty, r.sn)));
+    /* ty cs - (tx sn), the product rounded first */
+    v = fma(dup(ty), dup(r.cs), mul(t, dup(-r.sn)));
+}
+
+/* One FP32 record at the pixels px[0..P) of row py, in FP64 if its disc reaches the warp. */
+template <int OP, int P, int TYPE>
+__device__ __forceinline__ void eval32_record(const lt_rec32 &r, bool maybe_near, const lt_rec64 *recs64,
+                                              const lt_nie64 *nie, const double (&px)[P], double py, int kmap,
+                                              Acc32<P> &acc)
+{
+    constexpr bool packed = P == 2 && TYPE == 81;
+    float u[P], v[P];
+    f2 u2, v2;
+    if constexpr (packed) {
+        frame32x2(r, px, py, u2, v2);
+        u[0] = p2::lo(u2), u[1] = p2::hi(u2), v[0] = p2::lo(v2), v[1] = p2::hi(v2);
+    } else {
+        const float ty = __double2float_rn(__dsub_rn(py, r.y0));
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            const float tx = __double2float_rn(__dsub_rn(px[k], r.x0));
+            u[k] = __fmaf_rn(tx, r.cs, __fmul_rn(ty, r.sn));
+            v[k] = __fmaf_rn(ty, r.cs, -__fmul_rn(tx, r.sn));
         }
-        if (OP & OP_POT) acc.bp.a = add(acc.bp.a, pot32x2(r, u, v, n, t));
+    }
+    bool near = false;
+    if (maybe_near) {
+        /* the FP64 disc (an FP64 proxy record has rnear2 = +inf: every pixel) */
+#pragma unroll
+        for (int k = 0; k < P; k++) near |= __fmaf_rn(u[k], u[k], __fmul_rn(v[k], v[k])) < r.rnear2;
+        near = __any_sync(0xffffffffu, near);
+    }
+    if (near) {
+        const lt_rec64 &r64 = recs64[r.idx64];
+        const lt_nie64 &rn = nie[r.idx64];
+        const double w = kmap ? r64.w : 1.0;
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            if (OP & OP_HESS) add_hess64(acc, k, hess_term<TYPE>(r64, px[k], py, w));
+            if (OP & OP_GRAD) {
+                const double2 t = grad_term<TYPE>(rn, px[k], py);
+                acc.gx[k] = __dadd_rn(acc.gx[k], t.x);
+                acc.gy[k] = __dadd_rn(acc.gy[k], t.y);
+            }
+            if (OP & OP_POT) acc.psi[k] = __dadd_rn(acc.psi[k], pot_term<TYPE>(rn, px[k], py));
+        }
+    } else if constexpr (packed) {
+        add32x2<OP>(r, terms32x2<OP, true>(r, u2, v2), acc);
+    } else {
+        terms32<OP, P, TYPE>(r, u, v, acc);
     }
 }
 
 /* One chunk of FP32 records (at most 128) for the pixels px[0..P) of row py, the lane's
  * pixels (ix .. ix + P - 1, iy) of grid `a`.  Every record of an FP32C chunk has the same
- * Kmap weight. */
-template <int OP, int P, int TYPE>
+ * Kmap weight.  With U = 2 the terms of two cut dPIE records interleave and are added in their
+ * order (small grids, where one record's chain at a time leaves the SM idle). */
+template <int OP, int P, int TYPE, int U = 1>
 __device__ __forceinline__ void eval32_chunk(const lt_rec32 *recs, const lt_rec64 *recs64, const lt_nie64 *nie, int count,
                                              const double (&px)[P], double py, const GridArgs &a, int ix, int iy,
                                              Acc32<P> &acc)
@@ -401,52 +479,22 @@ __device__ __forceinline__ void eval32_chunk(const lt_rec32 *recs, const lt_rec6
         const uint64_t mask = near_mask(recs + h0, n, box);
 #pragma unroll 1
         for (int h = h0; h < h0 + n; h++) {
-            const lt_rec32 &r = recs[h];
-            constexpr bool packed = P == 2 && TYPE == 81;
-            float u[P], v[P];
-            f2 u2, v2;
-            const float ty = __double2float_rn(__dsub_rn(py, r.y0));
-            if constexpr (packed) {
-                using namespace p2;
-                const f2 t = pack(__double2float_rn(__dsub_rn(px[0], r.x0)), __double2float_rn(__dsub_rn(px[1], r.x0)));
-                u2 = fma(t, dup(r.cs), dup(__fmul_rn(ty, r.sn)));
-                /* ty cs - (tx sn), the product rounded first */
-                v2 = fma(dup(ty), dup(r.cs), mul(t, dup(-r.sn)));
-                u[0] = lo(u2), u[1] = hi(u2), v[0] = lo(v2), v[1] = hi(v2);
-            } else {
-#pragma unroll
-                for (int k = 0; k < P; k++) {
-                    const float tx = __double2float_rn(__dsub_rn(px[k], r.x0));
-                    u[k] = __fmaf_rn(tx, r.cs, __fmul_rn(ty, r.sn));
-                    v[k] = __fmaf_rn(ty, r.cs, -__fmul_rn(tx, r.sn));
+            if constexpr (U == 2 && P == 2 && TYPE == 81) {
+                if (h + 1 < h0 + n && ((mask >> (h - h0)) & 3ull) == 0) {
+                    f2 u[2], v[2];
+                    frame32x2(recs[h], px, py, u[0], v[0]);
+                    frame32x2(recs[h + 1], px, py, u[1], v[1]);
+                    const Terms2 t0 = terms32x2<OP, false>(recs[h], u[0], v[0]);
+                    const Terms2 t1 = terms32x2<OP, false>(recs[h + 1], u[1], v[1]);
+                    add32x2<OP>(recs[h], t0, acc);
+                    if ((h & (kBlock32 - 1)) == kBlock32 - 1) fold32<OP, P>(acc, wchunk);
+                    h++;
+                    add32x2<OP>(recs[h], t1, acc);
+                    if ((h & (kBlock32 - 1)) == kBlock32 - 1) fold32<OP, P>(acc, wchunk);
+                    continue;
                 }
             }
-            bool near = false;
-            if ((mask >> (h - h0)) & 1ull) {
-                /* the FP64 disc (an FP64 proxy record has rnear2 = +inf: every pixel) */
-#pragma unroll
-                for (int k = 0; k < P; k++) near |= __fmaf_rn(u[k], u[k], __fmul_rn(v[k], v[k])) < r.rnear2;
-                near = __any_sync(0xffffffffu, near);
-            }
-            if (near) {
-                const lt_rec64 &r64 = recs64[r.idx64];
-                const lt_nie64 &rn = nie[r.idx64];
-                const double w = kmap ? r64.w : 1.0;
-#pragma unroll
-                for (int k = 0; k < P; k++) {
-                    if (OP & OP_HESS) add_hess64(acc, k, hess_term<TYPE>(r64, px[k], py, w));
-                    if (OP & OP_GRAD) {
-                        const double2 t = grad_term<TYPE>(rn, px[k], py);
-                        acc.gx[k] = __dadd_rn(acc.gx[k], t.x);
-                        acc.gy[k] = __dadd_rn(acc.gy[k], t.y);
-                    }
-                    if (OP & OP_POT) acc.psi[k] = __dadd_rn(acc.psi[k], pot_term<TYPE>(rn, px[k], py));
-                }
-            } else if constexpr (packed) {
-                terms32x2<OP>(r, u2, v2, acc);
-            } else {
-                terms32<OP, P, TYPE>(r, u, v, acc);
-            }
+            eval32_record<OP, P, TYPE>(recs[h], (mask >> (h - h0)) & 1ull, recs64, nie, px, py, kmap, acc);
             if ((h & (kBlock32 - 1)) == kBlock32 - 1) fold32<OP, P>(acc, wchunk);
         }
     }

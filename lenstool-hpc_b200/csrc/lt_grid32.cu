@@ -136,12 +136,12 @@ struct C32Args {
     double mu_tol; /* recompute pixels whose FP32 error bound on mu exceeds this (0: none) */
 };
 
-/* Pass 1.  NT threads per CTA (8 lanes x P columns by 4 rows per warp, warps 4 across):
- * a tile is 32 P columns by NT / 32 rows; registers are cut for MINB resident CTAs per
+/* Pass 1.  NT threads per CTA (8 lanes x P columns by 4 rows per warp, warps 4 across, or 2 in
+ * CTAs of 64): a tile is 32 P columns by NT / 32 rows (16 P by 4); registers are cut for MINB resident CTAs per
  * SM.  Persistent CTAs stride over the tiles; for each tile the chunks of the catalogue
  * are staged into shared memory by cp.async.bulk, chunk k + 1 in flight while chunk k is
  * evaluated. */
-template <int OP, int P, int NT, int MINB>
+template <int OP, int P, int NT, int MINB, int U = 1>
 __global__ void __launch_bounds__(NT, MINB) grid32c_kernel(const C32Args A)
 {
     const GridArgs &a = A.g;
@@ -152,9 +152,10 @@ __global__ void __launch_bounds__(NT, MINB) grid32c_kernel(const C32Args A)
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    constexpr int kTileW = 32 * P, kTileH = NT / 32;
-    const int ox = (warp & 3) * (8 * P) + (lane & 7) * P;
-    const int oy = (warp >> 2) * 4 + (lane >> 3);
+    constexpr int kAcross = NT < 128 ? NT / 32 : 4; /* warps side by side */
+    constexpr int kTileW = kAcross * 8 * P, kTileH = NT / 32 / kAcross * 4;
+    const int ox = (warp % kAcross) * (8 * P) + (lane & 7) * P;
+    const int oy = (warp / kAcross) * 4 + (lane >> 3);
     const int my_tiles = (blockIdx.x < a.ntiles) ? (a.ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     const long steps = (long)my_tiles * A.nchunks;
 
@@ -216,9 +217,9 @@ __global__ void __launch_bounds__(NT, MINB) grid32c_kernel(const C32Args A)
         if (c.pad & CHUNK_FP32) {
             const lt_rec32 *recs = reinterpret_cast<const lt_rec32 *>(buf);
             switch (c.type) {
-            case 81: eval32_chunk<OP, P, 81>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc); break;
-            case 8: eval32_chunk<OP, P, 8>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc); break;
-            case 5: eval32_chunk<OP, P, 5>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc); break;
+            case 81: eval32_chunk<OP, P, 81, U>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc); break;
+            case 8: eval32_chunk<OP, P, 8, U>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc); break;
+            case 5: eval32_chunk<OP, P, 5, U>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc); break;
             default: break;
             }
         } else {
@@ -273,7 +274,10 @@ __global__ void __launch_bounds__(NT, MINB) grid32c_kernel(const C32Args A)
 using Kern32 = void (*)(const C32Args);
 
 /* The FP32C kernel shapes (pixels per thread, CTAs per SM, threads per CTA); the halo
- * stage size (records per chunk: 32, 64 or 128) is a launch argument. */
+ * stage size (records per chunk: 32, 64 or 128) is a launch argument.  The two-pixel shapes of 128
+ * threads take two records at a time: 300 halos on 2048^2, 256 threads and one record / 128
+ * threads and two, Hessian 3.24 / 3.02 ms, deflection 3.73 / 3.55, lens maps 6.02 / 6.38 (their
+ * one record has chains enough, two spill over the registers). */
 template <int OP>
 static Kern32 pick_shape32(int shape)
 {
@@ -284,9 +288,24 @@ static Kern32 pick_shape32(int shape)
     case LT_SHAPE(2, 2) & 0xffff: return grid32c_kernel<OP, 2, 256, 2>;
     case LT_SHAPE4(1, 2, 128, 64) & 0xffff: return grid32c_kernel<OP, 1, 128, 2>;
     case LT_SHAPE4(1, 4, 128, 64) & 0xffff: return grid32c_kernel<OP, 1, 128, 4>;
-    case LT_SHAPE4(2, 2, 128, 64) & 0xffff: return grid32c_kernel<OP, 2, 128, 2>;
-    case LT_SHAPE4(2, 3, 128, 64) & 0xffff: return grid32c_kernel<OP, 2, 128, 3>;
-    case LT_SHAPE4(2, 4, 128, 64) & 0xffff: return grid32c_kernel<OP, 2, 128, 4>;
+    case LT_SHAPE4(2, 2, 128, 64) & 0xffff: return grid32c_kernel<OP, 2, 128, 2, 2>;
+    case LT_SHAPE4(2, 3, 128, 64) & 0xffff: return grid32c_kernel<OP, 2, 128, 3, 2>;
+    case LT_SHAPE4(2, 4, 128, 64) & 0xffff: return grid32c_kernel<OP, 2, 128, 4, 2>;
+    default: return nullptr;
+    }
+}
+
+/* Small grids: CTAs of 64 threads, so that their few warps spread evenly over the SMs, two records
+ * at a time.  The warps' pixel boxes, and so the FP64 discs' decisions and every bit, are those of
+ * the other two-pixel shapes. */
+constexpr int kSmallThreads = 64;
+static Kern32 small_kernel32(int op)
+{
+    switch (op) {
+    case OP_HESS: return grid32c_kernel<OP_HESS, 2, kSmallThreads, 4, 2>;
+    case OP_POT: return grid32c_kernel<OP_POT, 2, kSmallThreads, 4, 2>;
+    case OP_HESS | OP_POT: return grid32c_kernel<OP_HESS | OP_POT, 2, kSmallThreads, 4, 2>;
+    case OP_GRAD: return grid32c_kernel<OP_GRAD, 2, kSmallThreads, 4, 2>;
     default: return nullptr;
     }
 }
@@ -351,12 +370,36 @@ static int launch_pass1(lt_context *ctx, const Fp32cCatalog &fc, int op, C32Args
     const int shape = ctx->shape[LT_FP32C][op & 7];
     Kern32 kern = pick_kernel32(op, shape);
     if (!kern) return (int)cudaErrorInvalidValue;
-    const int P = shape_ppt(shape), NT = shape_threads(shape), cap = shape_cap(shape);
+    const int P = shape_ppt(shape);
+    int NT = shape_threads(shape), cap = shape_cap(shape);
+    auto tiles = [&](int w, int h) {
+        A.g.tiles_x = (A.g.nx + w - 1) / w;
+        A.g.ntiles = A.g.tiles_x * ((A.g.ny + h - 1) / h);
+    };
+    tiles(32 * P, NT / 32);
+    /* Grids of few warps per scheduler (two-pixel shapes), 300 halos, us:
+     *   warps     Hessian 256 / 128 x 2 / 64 x 2     lens maps 256 / 128 x 2 (3 CTAs) / 64 x 2
+     *    1.3      85 / 74 / 72                       160 / 138 / 138
+     *    2.7      126 / 96 / 95                      236 / 187 / 217
+     *    5.5      241 / 195 / 178                    446 / 396 / 381
+     *    9.6      355 / 291 / 283                    658 / 608 / 622
+     *   16.9      582 / 487 / 510                    1074 / 1027 / 1090
+     *   27.7      818 / 763 / 788                    1518 / 1580 / 1709 */
+    const double warps = ((A.g.nx + 15) / 16) * (double)((A.g.ny + 3) / 4) / (4. * ctx->num_sms);
+    if (P == 2 && warps <= (op == (OP_HESS | OP_POT) ? 1.6 : 10.)) {
+        kern = small_kernel32(op);
+        NT = kSmallThreads;
+        cap = 64; /* 32 KB of stages */
+        tiles(32, 4);
+    } else if (P == 2 && op == (OP_HESS | OP_POT) && warps <= 17.) {
+        kern = pick_kernel32(op, LT_SHAPE4(2, 3, 128, 64));
+        NT = 128;
+        cap = 64;
+        tiles(64, 4);
+    }
     A.cap = cap;
     chunks_for_cap(fc, cap, &A.chunks, &A.nchunks);
     A.recs32 = fc.recs32;
-    A.g.tiles_x = (A.g.nx + 32 * P - 1) / (32 * P);
-    A.g.ntiles = A.g.tiles_x * ((A.g.ny + NT / 32 - 1) / (NT / 32));
     const size_t smem = 2 * (size_t)cap * sizeof(lt_rec64); /* allowed once by configure_kernels32 */
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);

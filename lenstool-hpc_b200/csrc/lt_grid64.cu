@@ -20,10 +20,11 @@
 
 namespace lt {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 256;      /* threads per CTA */
+constexpr int kSmallThreads = 64;  /* ... for small grids */
 
-template <int OP, int P, bool LIST, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a)
+template <int OP, int P, bool LIST, int MINB, int NT = kThreads, int U = 1>
+__global__ void __launch_bounds__(NT, MINB) grid64_kernel(const GridArgs a)
 {
     static_assert(!LIST || (OP == (OP_HESS | OP_NI)), "list mode: the FP64 recomputation's Hessian");
     extern __shared__ __align__(16) unsigned char smem[];
@@ -33,21 +34,29 @@ __global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    constexpr int kTileW = 32 * P;
-    const int ox = (warp & 3) * (8 * P) + (lane & 7) * P; /* pixel offset in the tile */
-    const int oy = (warp >> 2) * 4 + (lane >> 3);
+    constexpr int kAcross = NT < 128 ? NT / 32 : 4; /* warps side by side */
+    constexpr int kTileW = kAcross * 8 * P, kTileH = NT / 32 / kAcross * 4;
+    const int ox = (warp % kAcross) * (8 * P) + (lane & 7) * P; /* pixel offset in the tile */
+    const int oy = (warp / kAcross) * 4 + (lane >> 3);
 
     int ntiles = a.ntiles, nlist = 0;
+    /* list mode: every CTA takes the same share of the list, a multiple of 32 entries, in tiles of
+     * at most NT P entries: one entry a thread while they fit, else P */
+    int share = 0, first = 0, mine = 0, part = 0;
     if (LIST) {
         nlist = *a.list_count;
         nlist = nlist < a.list_cap ? nlist : a.list_cap;
-        ntiles = (nlist + kThreads * P - 1) / (kThreads * P);
+        share = (nlist + (int)gridDim.x - 1) / (int)gridDim.x;
+        share = (share + 31) / 32 * 32;
+        first = (int)blockIdx.x * share;
+        mine = nlist - first < share ? nlist - first : share;
         /* the count of recomputed pixels (lt_recompute_count): the 64-bit word 2 of the
          * context's status block */
         if (blockIdx.x == 0 && tid == 0 && a.status)
             atomicAdd(reinterpret_cast<unsigned long long *>(a.status + 2), (unsigned long long)nlist);
     }
-    const int my_tiles = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int my_tiles = LIST ? (mine > 0 ? (mine + NT * P - 1) / (NT * P) : 0)
+                              : ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     const long steps = (long)my_tiles * a.nchunks;
 
     if (tid == 0) {
@@ -81,13 +90,16 @@ __global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a
         if (ci == 0) {
             const int tile = blockIdx.x + (int)(s / a.nchunks) * gridDim.x;
             if (LIST) {
-                /* P list entries a thread, kThreads apart */
+                /* this tile's entries: the first `part` to entry k = 0 of the threads, the rest to k = 1 */
+                const int t0 = (int)(s / a.nchunks) * NT * P, left = mine - t0, count = left < NT * P ? left : NT * P;
+                part = count <= NT ? count : ((count + 1) / 2 + 31) / 32 * 32;
 #pragma unroll
                 for (int k = 0; k < P; k++) {
-                    const int e = (tile * P + k) * kThreads + tid;
-                    const int p = a.list[e < nlist ? e : nlist - 1];
+                    const int i = k * part + tid;
+                    const bool have = tid < part && i < count && (k == 0 || part < count);
+                    const int p = a.list[first + t0 + (have ? i : 0)];
                     lx[k] = p % a.nx;
-                    ly[k] = e < nlist ? p / a.nx : a.ny; /* rows >= ny are not stored */
+                    ly[k] = have ? p / a.nx : a.ny; /* rows >= ny are not stored */
                     px[k] = pixel_x(a, lx[k]);
                     lpy[k] = pixel_y(a, ly[k] < a.ny ? ly[k] : a.ny - 1);
                     acc.hxx[k] = acc.hyy[k] = acc.hxy[k] = 0.;
@@ -95,7 +107,7 @@ __global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a
             } else {
                 const int tx = tile % a.tiles_x, ty = tile / a.tiles_x;
                 ix = tx * kTileW + ox;
-                iy = ty * 8 + oy;
+                iy = ty * kTileH + oy;
                 const int cy = iy < a.ny ? iy : a.ny - 1;
                 py = pixel_y(a, cy);
 #pragma unroll
@@ -124,8 +136,20 @@ __global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a
         if (LIST) {
             /* the staged records are the closed-form records lt_nie64; acc.hxx, acc.hyy and
              * acc.hxy hold the convergence and shear sums */
-            eval_nie_chunk<P>(c, reinterpret_cast<const lt_nie64 *>(recs), px, lpy, a.kmap, acc.hxx, acc.hyy,
-                              acc.hxy);
+            const lt_nie64 *nie = reinterpret_cast<const lt_nie64 *>(recs);
+            const bool single = !__any_sync(0xffffffffu, ly[P - 1] < a.ny); /* warp-uniform */
+            if (!__any_sync(0xffffffffu, ly[0] < a.ny)) {
+                /* no entry in this warp */
+            } else if (single) { /* one pixel a thread, the chains of four records interleaved */
+                const double x1[1] = {px[0]}, y1[1] = {lpy[0]};
+                double k1[1] = {acc.hxx[0]}, g1[1] = {acc.hyy[0]}, g2[1] = {acc.hxy[0]};
+                eval_nie_chunk<1, 4>(c, nie, x1, y1, a.kmap, k1, g1, g2);
+                acc.hxx[0] = k1[0];
+                acc.hyy[0] = g1[0];
+                acc.hxy[0] = g2[0];
+            } else {
+                eval_nie_chunk<P>(c, nie, px, lpy, a.kmap, acc.hxx, acc.hyy, acc.hxy);
+            }
             if (ci == a.nchunks - 1) {
 #pragma unroll
                 for (int k = 0; k < P; k++) {
@@ -140,7 +164,7 @@ __global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a
             __syncthreads(); /* buffer b is refilled by the copy issued at step s + 1 */
             continue;
         }
-        eval_any64<OP, P>(c, recs, px, py, a.kmap, acc);
+        eval_any64<OP, P, U>(c, recs, px, py, a.kmap, acc);
         if ((OP & OP_HEX) && (c.pad & CHUNK_RUN_END))
             close_run64<OP, P>(acc, a.kmap, reinterpret_cast<const lt_rec64 *>(recs)[c.count - 1].w);
 
@@ -172,27 +196,32 @@ __global__ void __launch_bounds__(kThreads, MINB) grid64_kernel(const GridArgs a
 
 /* Launch one shape: P pixels per thread, registers cut for MINB resident CTAs per SM.
  * Tiles are (32 P) x 8 pixels; persistent grid of (resident CTAs per SM) x SMs. */
-template <int OP, int P, bool LIST, int MINB>
+template <int OP, int P, bool LIST, int MINB, int NT = kThreads, int U = 1>
 static int launch_op(const GridArgs &args, int num_sms, cudaStream_t stream)
 {
     const size_t smem = 2 * LT_CHUNK * sizeof(lt_rec64);
-    auto kern = grid64_kernel<OP, P, LIST, MINB>;
+    auto kern = grid64_kernel<OP, P, LIST, MINB, NT, U>;
+    constexpr int across = NT < 128 ? NT / 32 : 4, w = across * 8 * P, h = NT / 32 / across * 4;
     GridArgs a = args;
-    a.tiles_x = (a.nx + 32 * P - 1) / (32 * P);
-    a.ntiles = a.tiles_x * ((a.ny + 7) / 8);
+    a.tiles_x = (a.nx + w - 1) / w;
+    a.ntiles = a.tiles_x * ((a.ny + h - 1) / h);
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);
     if (per_sm < 1) per_sm = 1;
     int blocks = num_sms * per_sm;
     if (!LIST && blocks > a.ntiles) blocks = a.ntiles;
     if (blocks < 1) blocks = 1;
-    kern<<<blocks, kThreads, smem, stream>>>(a);
+    kern<<<blocks, NT, smem, stream>>>(a);
     return (int)cudaGetLastError();
 }
 
 template <int OP>
 static int launch_shape(int shape, const GridArgs &a, int num_sms, cudaStream_t s)
 {
+    /* a grid of less than two CTAs an SM: CTAs of 64 threads, one pixel each, so that it spreads
+     * over all SMs, and (reference-order Hessian) two records a thread at a time */
+    if ((long)((a.nx + 31) / 32) * ((a.ny + 7) / 8) < 2 * num_sms)
+        return launch_op<OP, 1, false, 4, kSmallThreads, 2>(a, num_sms, s);
     switch (shape) {
     case LT_SHAPE(1, 1): return launch_op<OP, 1, false, 1>(a, num_sms, s);
     case LT_SHAPE(1, 2): return launch_op<OP, 1, false, 2>(a, num_sms, s);

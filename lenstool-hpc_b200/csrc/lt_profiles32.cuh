@@ -390,27 +390,30 @@ __device__ __forceinline__ f2 fatanh_third2(f2 s)
     return mul(s, p);
 }
 
-/* fatanh_any of both halves.  Galaxies mostly stay within |y| <= 1/3: the logarithm (an
- * approximate reciprocal and an approximate log2 a pixel) is left out where the whole warp does. */
+/* fatanh_any of both halves.  Galaxies mostly stay within |y| <= 1/3: with SKIP the logarithm (an
+ * approximate reciprocal and an approximate log2 a pixel) is left out where the whole warp does;
+ * without it no branch keeps two records' chains from interleaving. */
+template <bool SKIP>
 __device__ __forceinline__ f2 fatanh_any2(f2 y)
 {
     using namespace p2;
     const bool b0 = fabsf(lo(y)) <= (1.f / 3.f), b1 = fabsf(hi(y)) <= (1.f / 3.f);
     f2 r = fatanh_third2(y);
-    if (__any_sync(0xffffffffu, !(b0 && b1)))
+    if (!SKIP || __any_sync(0xffffffffu, !(b0 && b1)))
         r = pack(b0 ? lo(r) : fhalf_log(f32::mul(f32::add(1.f, lo(y)), frcp(f32::sub(1.f, lo(y))))),
                  b1 ? hi(r) : fhalf_log(f32::mul(f32::add(1.f, hi(y)), frcp(f32::sub(1.f, hi(y))))));
     return r;
 }
 
-/* half_log1p_pos of both halves: one of the two forms where the whole warp takes it (a halo's
- * cut radius mostly has the warp's pixels on one side). */
+/* half_log1p_pos of both halves: with SKIP only one of the two forms where the whole warp takes
+ * it (a halo's cut radius mostly has the warp's pixels on one side). */
+template <bool SKIP>
 __device__ __forceinline__ f2 half_log1p_pos2(f2 t)
 {
     using namespace p2;
     const bool b0 = lo(t) <= 1.f, b1 = hi(t) <= 1.f;
     f2 r, g;
-    const bool small = __any_sync(0xffffffffu, b0 || b1), large = __any_sync(0xffffffffu, !(b0 && b1));
+    const bool small = !SKIP || __any_sync(0xffffffffu, b0 || b1), large = !SKIP || __any_sync(0xffffffffu, !(b0 && b1));
     if (large) {
         const f2 w = add(dup(1.f), t);
         g = mul(pack(flog2(lo(w)), flog2(hi(w))), dup(kHalfLn2f));
@@ -467,6 +470,7 @@ __device__ __forceinline__ KG2 hess32x2(const lt_rec32 &h, f2 u, f2 v, const Nie
     return r;
 }
 
+template <bool SKIP>
 __device__ __forceinline__ G2 grad32x2(const lt_rec32 &h, f2 u, f2 v, const Nie2 &n)
 {
     using namespace p2;
@@ -475,9 +479,10 @@ __device__ __forceinline__ G2 grad32x2(const lt_rec32 &h, f2 u, f2 v, const Nie2
     const f2 du = fma(dup(h.k2), n.uu, mul(add(n.pc, dup(h.sc)), add(n.pt, dup(h.st))));
     const f2 nv = mul(mul(nk, v), add(n.dpsi, dup(h.dsq2)));
     const f2 dv = fma(dup(-h.k2), n.vv, mul(add(n.pc, dup(h.q2sc)), add(n.pt, dup(h.q2st))));
-    return {mul(dup(h.Ak), fatan_pos2(nu, du)), mul(dup(h.Ak), fatanh_any2(mul(nv, frcp2(dv))))};
+    return {mul(dup(h.Ak), fatan_pos2(nu, du)), mul(dup(h.Ak), fatanh_any2<SKIP>(mul(nv, frcp2(dv))))};
 }
 
+template <bool SKIP>
 __device__ __forceinline__ f2 pot32x2(const lt_rec32 &h, f2 u, f2 v, const Nie2 &n, const G2 &g)
 {
     using namespace p2;
@@ -487,7 +492,7 @@ __device__ __forceinline__ f2 pot32x2(const lt_rec32 &h, f2 u, f2 v, const Nie2 
     const f2 opt_c = mul(fma(dup(h.k2), n.uu, mul(pcs, pcs)), dup(h.i4rc2));
     const f2 tt = mul(fma(mul(dup(h.tst), n.B), frcp2(add(n.pt, dup(h.qst))), r2), dup(h.i4rcut2));
     const f2 lc = pack(flog2(lo(opt_c)), flog2(hi(opt_c)));
-    return sub(xa, fma(dup(h.Ascl2), lc, mul(dup(-2.f * h.Ast), half_log1p_pos2(tt))));
+    return sub(xa, fma(dup(h.Ascl2), lc, mul(dup(-2.f * h.Ast), half_log1p_pos2<SKIP>(tt))));
 }
 
 /* Potential of one pair from its deflection g (halo frame):

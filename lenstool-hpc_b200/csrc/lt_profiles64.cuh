@@ -341,32 +341,41 @@ __device__ __forceinline__ bool hess_frame(const lt_rec64 &h, double u, double v
     return !odd.any();
 }
 
-/* One halo's Hessians at P pixels of a row added to the run accumulators.  220 FP64 operations
- * a dPIE pair; the odd operands' branch is taken once in ~10^9 pairs. */
-template <int TYPE, int P>
-__device__ __forceinline__ void hess_pairs(const lt_rec64 &h, const double (&px)[P], double py, Mat (&acc)[P])
+/* The Hessians of U records at P pixels of a row added, in their order, to the run accumulators.
+ * 220 FP64 operations a dPIE pair; the odd operands' branch is taken once in ~10^9 pairs.  The
+ * U P pairs are independent chains that interleave (U = 2 where a grid is too small to fill the
+ * SMs with warps). */
+template <int TYPE, int P, int U>
+__device__ __forceinline__ void hess_pairs(const lt_rec64 *h, const double (&px)[P], double py, Mat (&acc)[P])
 {
-    const double ty = S(py, h.y0);
-    double u[P], v[P];
-    Mat m[P];
+    double u[U][P], v[U][P];
+    Mat m[U][P];
     bool ok = true;
 #pragma unroll
-    for (int k = 0; k < P; k++) {
-        const double tx = S(px[k], h.x0);
-        u[k] = A(M(tx, h.cs), M(ty, h.sn));
-        v[k] = S(M(ty, h.cs), M(tx, h.sn));
-        ok &= hess_frame<TYPE>(h, u[k], v[k], m[k]);
+    for (int i = 0; i < U; i++) {
+        const double ty = S(py, h[i].y0);
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            const double tx = S(px[k], h[i].x0);
+            u[i][k] = A(M(tx, h[i].cs), M(ty, h[i].sn));
+            v[i][k] = S(M(ty, h[i].cs), M(tx, h[i].sn));
+            ok &= hess_frame<TYPE>(h[i], u[i][k], v[i][k], m[i][k]);
+        }
     }
     if (TYPE != 5 && !ok) {
 #pragma unroll
-        for (int k = 0; k < P; k++) {
-            Mat t;
-            hess_ieee<TYPE>(h, u[k], v[k], t);
-            m[k] = t;
-        }
+        for (int i = 0; i < U; i++)
+#pragma unroll
+            for (int k = 0; k < P; k++) {
+                Mat t;
+                hess_ieee<TYPE>(h[i], u[i][k], v[i][k], t);
+                m[i][k] = t;
+            }
     }
 #pragma unroll
-    for (int k = 0; k < P; k++) rotate_acc(m[k], h.cs, h.sn, acc[k]);
+    for (int i = 0; i < U; i++)
+#pragma unroll
+        for (int k = 0; k < P; k++) rotate_acc(m[i][k], h[i].cs, h[i].sn, acc[k]);
 }
 } // namespace ex
 
