@@ -262,8 +262,9 @@ lt_status lt_get_kernel_shape(const lt_context *ctx, int32_t precision, int32_t 
                               int32_t *ctas_per_sm);
 /* The full kernel configuration: besides the shape, the threads per CTA (128 or 256; a
  * tile is 32 x pixels_per_thread columns by threads / 32 rows) and the halo records per
- * shared-memory stage (32, 64 or 128).  LT_FP32C kernels come in the shapes
- * (pixels, CTAs/SM, threads) = (1|2, 1|2, 256), (1, 2|4, 128), (2, 2|3|4, 128), each with
+ * shared-memory stage (32, 64 or 128).  Grids too small to fill the SMs run in CTAs of 64
+ * or 128 threads whatever the configuration says, with the same planes.  LT_FP32C kernels
+ * come in the shapes (pixels, CTAs/SM, threads) = (1|2, 1|2, 256), (1, 2|4, 128), (2, 2|3|4, 128), each with
  * every stage size; the FP64 kernels in their four 256-thread, 64-record shapes.  An
  * unbuilt configuration is LT_ERR_INVALID_ARGUMENT.  lt_set_kernel_shape keeps 256 threads
  * and 64-record stages. */

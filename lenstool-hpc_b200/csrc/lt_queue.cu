@@ -210,7 +210,7 @@ __device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_
                                   const lt_rec32 *recs = reinterpret_cast<const lt_rec32 *>(buf);
                                   switch (c.type) {
                                   case 81:
-                                      eval32_chunk<OP, P, 81>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
+                                      eval32_chunk<OP, P, 81, OP == (OP_HESS | OP_POT) ? 1 : 2>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
                                       break;
                                   case 8:
                                       eval32_chunk<OP, P, 8>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
@@ -305,7 +305,7 @@ __device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_
                                      if (!have[0]) return;
                                      const lt_nie64 *recs = reinterpret_cast<const lt_nie64 *>(buf);
                                      if (one)
-                                         eval_nie_chunk<1>(c, recs, px1, py1, a.kmap, kap1, g11, g21);
+                                         eval_nie_chunk<1, 4>(c, recs, px1, py1, a.kmap, kap1, g11, g21);
                                      else
                                          eval_nie_chunk<P>(c, recs, qpx, qpy, a.kmap, kap, g1, g2);
                                  });
