@@ -622,7 +622,7 @@ int lt::launch_fp64(lt_context *ctx, const lt_catalog *cat, int op, int precisio
         a.out[0] = a.out[pot];
         op = OP_POT;
     }
-    if (side) return launch_tree64(cat, op, a, side, ctx->num_sms, stream);
+    if (side) return launch_tree64(cat, op, a, side, stream);
     return launch_grid64_tiled(op, a, ctx->num_sms, stream, ctx->shape[precision][op & 7]);
 }
 

@@ -117,7 +117,7 @@ lt_status run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g, int
 int tree_tables();
 int configure_tree64();
 int tree_side(const lt_catalog *cat, int op, int nx, int ny, double dx, double dy, int num_sms);
-int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side, int num_sms, void *stream);
+int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side, void *stream);
 /* FP64 sums `op` of one precision on a grid or a band of one; `side`: tree_side of the whole grid */
 int launch_fp64(lt_context *ctx, const lt_catalog *cat, int op, int precision, GridArgs &a, int side, void *stream);
 /* the tile side of a call's closed-form sums (0: direct) */

@@ -24,7 +24,10 @@
  * through shared memory (cp.async.bulk, two 64-record stages), then two pixels a pass while the
  * near records, gathered in shared memory, are walked.  Between them the node values are
  * contracted along y for the rows of a pass and along x for each pixel: 17 FP64 operations a
- * pixel and plane.  Bound by the FP64 pipe like the direct kernels.
+ * pixel and plane.  A tile's time is a latency chain (8 warps, one node a thread), so far records
+ * go two at a time: 410 -> 360 us for the deflection of 200 halos on 1024^2 with the rows of
+ * tiles launched from the middle outwards, where most halos are, one CTA each (tiles strided over
+ * resident CTAs left SMs idle for 26% of the time).
  */
 #include <cmath>
 #include <cuda_runtime.h>
@@ -122,6 +125,33 @@ __device__ __forceinline__ void tree_any(int type, const lt_nie64 &r, const doub
     }
 }
 
+/* Two records at one point: two chains that interleave, added in their order. */
+template <int OP>
+__device__ __forceinline__ void tree_two(int type, const lt_nie64 &r0, const lt_nie64 &r1, const double (&px)[1],
+                                         const double (&py)[1], int kmap, double (&s)[1][TreeOp<OP>::planes])
+{
+    double t[2][1][TreeOp<OP>::planes];
+#pragma unroll
+    for (int q = 0; q < TreeOp<OP>::planes; q++) t[0][0][q] = t[1][0][q] = 0.;
+    switch (type) {
+    case 81:
+        tree_pair<OP, 81, 1>(r0, px, py, kmap, t[0]);
+        tree_pair<OP, 81, 1>(r1, px, py, kmap, t[1]);
+        break;
+    case 8:
+        tree_pair<OP, 8, 1>(r0, px, py, kmap, t[0]);
+        tree_pair<OP, 8, 1>(r1, px, py, kmap, t[1]);
+        break;
+    case 5:
+        tree_pair<OP, 5, 1>(r0, px, py, kmap, t[0]);
+        tree_pair<OP, 5, 1>(r1, px, py, kmap, t[1]);
+        break;
+    default: break;
+    }
+#pragma unroll
+    for (int q = 0; q < TreeOp<OP>::planes; q++) s[0][q] += t[0][0][q] + t[1][0][q];
+}
+
 template <int OP>
 __global__ void __launch_bounds__(kTreeThreads, 2) tree64_kernel(const TreeArgs A)
 {
@@ -158,172 +188,175 @@ __global__ void __launch_bounds__(kTreeThreads, 2) tree64_kernel(const TreeArgs 
                  &bars[ci & 1]);
     };
 
-    for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
-        const int tx0 = (tile % a.tiles_x) * T, ty0 = (tile / a.tiles_x) * T;
-        const double x0 = pixel_x(a, tx0), x1 = pixel_x(a, tx0 + T - 1);
-        const double y0 = pixel_y(a, ty0), y1 = pixel_y(a, ty0 + T - 1);
-        const double xc = 0.5 * (x0 + x1), yc = 0.5 * (y0 + y1), hx = 0.5 * (x1 - x0), hy = 0.5 * (y1 - y0);
-        const double diag = sqrt(hx * hx + hy * hy), reach = TreeOp<OP>::far * fmax(fabs(hx), fabs(hy));
+    /* rows of tiles from the middle outwards: the halos crowd there, and the dear tiles go first */
+    const int trows = a.ntiles / a.tiles_x, mid = (trows - 1) / 2;
+    const int r = (int)blockIdx.x / a.tiles_x, row = mid + ((r & 1) ? (r + 1) / 2 : -(r / 2));
+    const int tx0 = ((int)blockIdx.x % a.tiles_x) * T, ty0 = row * T;
+    const double x0 = pixel_x(a, tx0), x1 = pixel_x(a, tx0 + T - 1);
+    const double y0 = pixel_y(a, ty0), y1 = pixel_y(a, ty0 + T - 1);
+    const double xc = 0.5 * (x0 + x1), yc = 0.5 * (y0 + y1), hx = 0.5 * (x1 - x0), hy = 0.5 * (y1 - y0);
+    const double diag = sqrt(hx * hx + hy * hy), reach = TreeOp<OP>::far * fmax(fabs(hx), fabs(hy));
 
-        /* the walk: near halos to the list, far ones summed at this thread's node */
-        double f[1][NQ];
+    /* the walk: near halos to the list, far ones summed at this thread's node */
+    double f[1][NQ];
 #pragma unroll
-        for (int q = 0; q < NQ; q++) f[0][q] = 0.;
-        const double nx[1] = {fma(hx, node_x, xc)}, ny[1] = {fma(hy, node_y, yc)};
-        int nlist = 0; /* warp 0's count of near halos */
-        if (tid == 0) issue(0);
-        for (int ci = 0; ci < a.nchunks; ci++) {
-            const int b = ci & 1;
-            if (tid == 0 && ci + 1 < a.nchunks) issue(ci + 1);
-            if (!wait_tile(&bars[b], phase[b], a.status)) {
-                if (tid == 0 && ci + 1 < a.nchunks) drain_tile(&bars[b ^ 1], phase[b ^ 1]);
-                return;
-            }
-            phase[b] ^= 1;
-            const lt_chunk c = a.chunks[ci];
-            const lt_nie64 *recs = stage + b * LT_CHUNK;
-            if (tid < 32) { /* one warp, so that the list keeps the catalogue's order */
-#pragma unroll
-                for (int w = 0; w < 2; w++) {
-                    const int i = 32 * w + tid;
-                    bool far = false;
-                    if (i < c.count) {
-                        const lt_nie64 &r = recs[i];
-                        const double dx = r.x0 - xc, dy = r.y0 - yc;
-                        const double d = fmax(sqrt(dx * dx + dy * dy) - diag, 0.);
-                        const double s = c.type == 5 ? 0. : r.sc;
-                        far = (c.type == 5 ? r.q2 / r.k : r.q2) * (d * d + s * s) >= reach * reach;
-                    }
-                    const uint32_t m = __ballot_sync(0xffffffffu, far);
-                    const uint32_t near = __ballot_sync(0xffffffffu, i < c.count && !far);
-                    const int at = nlist + __popc(near & ((1u << tid) - 1u));
-                    if (i < c.count && !far && at < kNearList) list[at] = c.start + i;
-                    nlist += __popc(near);
-                    if (tid == 0) s_far[w] = m;
-                }
-            }
-            __syncthreads();
-            double fc[1][NQ]; /* the chunk's own sum: fewer roundings of the large total */
-#pragma unroll
-            for (int q = 0; q < NQ; q++) fc[0][q] = 0.;
-#pragma unroll 1
-            for (int w = 0; w < 2; w++)
-                for (uint32_t m = s_far[w]; m; m &= m - 1)
-                    tree_any<OP, 1>(c.type, recs[32 * w + __ffs(m) - 1], nx, ny, a.kmap, fc);
-#pragma unroll
-            for (int q = 0; q < NQ; q++) f[0][q] += fc[0][q];
-            __syncthreads(); /* the stage and s_far are refilled */
+    for (int q = 0; q < NQ; q++) f[0][q] = 0.;
+    const double nx[1] = {fma(hx, node_x, xc)}, ny[1] = {fma(hy, node_y, yc)};
+    int nlist = 0; /* warp 0's count of near halos */
+    if (tid == 0) issue(0);
+    for (int ci = 0; ci < a.nchunks; ci++) {
+        const int b = ci & 1;
+        if (tid == 0 && ci + 1 < a.nchunks) issue(ci + 1);
+        if (!wait_tile(&bars[b], phase[b], a.status)) {
+            if (tid == 0 && ci + 1 < a.nchunks) drain_tile(&bars[b ^ 1], phase[b ^ 1]);
+            return;
         }
+        phase[b] ^= 1;
+        const lt_chunk c = a.chunks[ci];
+        const lt_nie64 *recs = stage + b * LT_CHUNK;
+        if (tid < 32) { /* one warp, so that the list keeps the catalogue's order */
 #pragma unroll
-        for (int q = 0; q < NQ; q++) F[q * kNodes * kNodes + tid] = f[0][q];
-        if (tid == 0) s_near = nlist;
+            for (int w = 0; w < 2; w++) {
+                const int i = 32 * w + tid;
+                bool far = false;
+                if (i < c.count) {
+                    const lt_nie64 &r = recs[i];
+                    const double dx = r.x0 - xc, dy = r.y0 - yc;
+                    const double d = fmax(sqrt(dx * dx + dy * dy) - diag, 0.);
+                    const double s = c.type == 5 ? 0. : r.sc;
+                    far = (c.type == 5 ? r.q2 / r.k : r.q2) * (d * d + s * s) >= reach * reach;
+                }
+                const uint32_t m = __ballot_sync(0xffffffffu, far);
+                const uint32_t near = __ballot_sync(0xffffffffu, i < c.count && !far);
+                const int at = nlist + __popc(near & ((1u << tid) - 1u));
+                if (i < c.count && !far && at < kNearList) list[at] = c.start + i;
+                nlist += __popc(near);
+                if (tid == 0) s_far[w] = m;
+            }
+        }
         __syncthreads();
-        int near = s_near;
-        const bool all = near > kNearList; /* more than the list holds: every halo at every pixel */
-        if (all) near = A.nhalos;
-        auto gather = [&](int i0, int n) { /* near records i0 .. i0 + n - 1 */
-            for (int e = tid; e < n * (int)(sizeof(lt_nie64) / 16); e += kTreeThreads) {
-                const int i = i0 + e / (int)(sizeof(lt_nie64) / 16);
-                const int4 *src = reinterpret_cast<const int4 *>(a.nie + (all ? i : list[i]));
-                reinterpret_cast<int4 *>(stage)[e] = src[e % (int)(sizeof(lt_nie64) / 16)];
-            }
-            for (int e = tid; e < n; e += kTreeThreads) s_type[e] = A.types[all ? i0 + e : list[i0 + e]];
-        };
-        if (near <= kNearStage) gather(0, near);
+        double fc[1][NQ]; /* the chunk's own sum: fewer roundings of the large total */
+#pragma unroll
+        for (int q = 0; q < NQ; q++) fc[0][q] = 0.;
+#pragma unroll 1
+        for (uint64_t m = (uint64_t)s_far[1] << 32 | s_far[0]; m;) { /* two records at a time */
+            const int i = __ffsll(m) - 1;
+            m &= m - 1;
+            const int j = m ? __ffsll(m) - 1 : -1;
+            m &= m - 1;
+            if (j >= 0)
+                tree_two<OP>(c.type, recs[i], recs[j], nx, ny, a.kmap, fc);
+            else
+                tree_any<OP, 1>(c.type, recs[i], nx, ny, a.kmap, fc);
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; q++) f[0][q] += fc[0][q];
+        __syncthreads(); /* the stage and s_far are refilled */
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; q++) F[q * kNodes * kNodes + tid] = f[0][q];
+    if (tid == 0) s_near = nlist;
+    __syncthreads();
+    int near = s_near;
+    const bool all = near > kNearList; /* more than the list holds: every halo at every pixel */
+    if (all) near = A.nhalos;
+    auto gather = [&](int i0, int n) { /* near records i0 .. i0 + n - 1 */
+        for (int e = tid; e < n * (int)(sizeof(lt_nie64) / 16); e += kTreeThreads) {
+            const int i = i0 + e / (int)(sizeof(lt_nie64) / 16);
+            const int4 *src = reinterpret_cast<const int4 *>(a.nie + (all ? i : list[i]));
+            reinterpret_cast<int4 *>(stage)[e] = src[e % (int)(sizeof(lt_nie64) / 16)];
+        }
+        for (int e = tid; e < n; e += kTreeThreads) s_type[e] = A.types[all ? i0 + e : list[i0 + e]];
+    };
+    if (near <= kNearStage) gather(0, near);
 
-        for (int r0 = 0; r0 < T && ty0 + r0 < a.ny; r0 += rows) {
-            __syncthreads(); /* F and the gathered records; H is free */
-            for (int e = tid; e < NQ * rows * kNodes; e += kTreeThreads) {
-                const int q = e / (rows * kNodes), r = (e / kNodes) % rows, i = e % kNodes;
-                const int row = r0 + r < T ? r0 + r : T - 1;
-                double h = 0.;
+    for (int r0 = 0; r0 < T && ty0 + r0 < a.ny; r0 += rows) {
+        __syncthreads(); /* F and the gathered records; H is free */
+        for (int e = tid; e < NQ * rows * kNodes; e += kTreeThreads) {
+            const int q = e / (rows * kNodes), r = (e / kNodes) % rows, i = e % kNodes;
+            const int row = r0 + r < T ? r0 + r : T - 1;
+            double h = 0.;
 #pragma unroll
-                for (int j = 0; j < kNodes; j++) h = fma(L[j * T + row], F[q * kNodes * kNodes + j * kNodes + i], h);
-                H[e] = h;
+            for (int j = 0; j < kNodes; j++) h = fma(L[j * T + row], F[q * kNodes * kNodes + j * kNodes + i], h);
+            H[e] = h;
+        }
+        double px[2], py[2], s[2][NQ];
+        int ix[2], iy[2], rr[2], cc[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int p = tid + k * kTreeThreads;
+            rr[k] = p / T;
+            cc[k] = p % T;
+            ix[k] = tx0 + cc[k];
+            iy[k] = rr[k] < rows && r0 + rr[k] < T ? ty0 + r0 + rr[k] : a.ny; /* >= ny: no pixel */
+            if (rr[k] >= rows) rr[k] = 0;
+            px[k] = pixel_x(a, ix[k] < a.nx ? ix[k] : a.nx - 1);
+            py[k] = pixel_y(a, iy[k] < a.ny ? iy[k] : a.ny - 1);
+#pragma unroll
+            for (int q = 0; q < NQ; q++) s[k][q] = 0.;
+        }
+        for (int i0 = 0; i0 < near; i0 += kNearStage) {
+            const int n = near - i0 < kNearStage ? near - i0 : kNearStage;
+            if (near > kNearStage) {
+                __syncthreads();
+                gather(i0, n);
+                __syncthreads();
             }
-            double px[2], py[2], s[2][NQ];
-            int ix[2], iy[2], rr[2], cc[2];
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const int p = tid + k * kTreeThreads;
-                rr[k] = p / T;
-                cc[k] = p % T;
-                ix[k] = tx0 + cc[k];
-                iy[k] = rr[k] < rows && r0 + rr[k] < T ? ty0 + r0 + rr[k] : a.ny; /* >= ny: no pixel */
-                if (rr[k] >= rows) rr[k] = 0;
-                px[k] = pixel_x(a, ix[k] < a.nx ? ix[k] : a.nx - 1);
-                py[k] = pixel_y(a, iy[k] < a.ny ? iy[k] : a.ny - 1);
-#pragma unroll
-                for (int q = 0; q < NQ; q++) s[k][q] = 0.;
-            }
-            for (int i0 = 0; i0 < near; i0 += kNearStage) {
-                const int n = near - i0 < kNearStage ? near - i0 : kNearStage;
-                if (near > kNearStage) {
-                    __syncthreads();
-                    gather(i0, n);
-                    __syncthreads();
-                }
 #pragma unroll 1
-                for (int b = 0; b < n; b += kNearBlock) { /* sums of blocks, as the chunks above */
-                    double sb[2][NQ];
+            for (int b = 0; b < n; b += kNearBlock) { /* sums of blocks, as the chunks above */
+                double sb[2][NQ];
 #pragma unroll
-                    for (int q = 0; q < NQ; q++) sb[0][q] = sb[1][q] = 0.;
+                for (int q = 0; q < NQ; q++) sb[0][q] = sb[1][q] = 0.;
 #pragma unroll 1
-                    for (int i = b; i < n && i < b + kNearBlock; i++)
-                        tree_any<OP, 2>(s_type[i], stage[i], px, py, a.kmap, sb);
+                for (int i = b; i < n && i < b + kNearBlock; i++)
+                    tree_any<OP, 2>(s_type[i], stage[i], px, py, a.kmap, sb);
 #pragma unroll
-                    for (int q = 0; q < NQ; q++) {
-                        s[0][q] += sb[0][q];
-                        s[1][q] += sb[1][q];
-                    }
+                for (int q = 0; q < NQ; q++) {
+                    s[0][q] += sb[0][q];
+                    s[1][q] += sb[1][q];
                 }
-            }
-            __syncthreads(); /* H */
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                if (all) continue;
-                double t[NQ];
-#pragma unroll
-                for (int q = 0; q < NQ; q++) t[q] = 0.;
-#pragma unroll
-                for (int i = 0; i < kNodes; i++) {
-                    const double l = L[i * T + cc[k]];
-#pragma unroll
-                    for (int q = 0; q < NQ; q++) t[q] = fma(l, H[(q * rows + rr[k]) * kNodes + i], t[q]);
-                }
-#pragma unroll
-                for (int q = 0; q < NQ; q++) s[k][q] += t[q];
-            }
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                if (ix[k] >= a.nx || iy[k] >= a.ny) continue;
-                constexpr int kh = OP & OP_GRAD ? 2 : 0, kp = kh + (OP & OP_HESS ? 3 : 0);
-                double hxx = 0., hyy = 0., hxy = 0.;
-                if (OP & OP_HESS) nie_hessian(s[k][kh], s[k][(kh + 1) % NQ], s[k][(kh + 2) % NQ], hxx, hyy, hxy);
-                const long pix = (long)iy[k] * a.nx + ix[k];
-                for (int o = 0; o < a.nout; o++)
-                    a.out[o][pix] = map_value4(a.kinds[o], OP & OP_GRAD ? s[k][0] : 0., OP & OP_GRAD ? s[k][1 % NQ] : 0.,
-                                               hxx, hyy, hxy, hxy, OP & OP_POT ? s[k][kp % NQ] : 0., a.D, a.mult, a.scale);
             }
         }
-        __syncthreads(); /* the stages and the list are refilled */
+        __syncthreads(); /* H */
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if (all) continue;
+            double t[NQ];
+#pragma unroll
+            for (int q = 0; q < NQ; q++) t[q] = 0.;
+#pragma unroll
+            for (int i = 0; i < kNodes; i++) {
+                const double l = L[i * T + cc[k]];
+#pragma unroll
+                for (int q = 0; q < NQ; q++) t[q] = fma(l, H[(q * rows + rr[k]) * kNodes + i], t[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < NQ; q++) s[k][q] += t[q];
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if (ix[k] >= a.nx || iy[k] >= a.ny) continue;
+            constexpr int kh = OP & OP_GRAD ? 2 : 0, kp = kh + (OP & OP_HESS ? 3 : 0);
+            double hxx = 0., hyy = 0., hxy = 0.;
+            if (OP & OP_HESS) nie_hessian(s[k][kh], s[k][(kh + 1) % NQ], s[k][(kh + 2) % NQ], hxx, hyy, hxy);
+            const long pix = (long)iy[k] * a.nx + ix[k];
+            for (int o = 0; o < a.nout; o++)
+                a.out[o][pix] = map_value4(a.kinds[o], OP & OP_GRAD ? s[k][0] : 0., OP & OP_GRAD ? s[k][1 % NQ] : 0.,
+                                           hxx, hyy, hxy, hxy, OP & OP_POT ? s[k][kp % NQ] : 0., a.D, a.mult, a.scale);
+        }
     }
 }
 
 template <int OP>
-static int launch_tree_op(TreeArgs &A, int num_sms, cudaStream_t s)
+static int launch_tree_op(TreeArgs &A, cudaStream_t s)
 {
     const size_t smem = tree_smem<OP>(A.T);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tree64_kernel<OP>, kTreeThreads, smem);
-    int blocks = num_sms * (per_sm < 1 ? 1 : per_sm);
-    if (blocks > A.g.ntiles) blocks = A.g.ntiles;
-    tree64_kernel<OP><<<blocks, kTreeThreads, smem, s>>>(A);
+    tree64_kernel<OP><<<A.g.ntiles, kTreeThreads, smem, s>>>(A);
     count_launch(1);
     return (int)cudaGetLastError();
 }
 
-int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side, int num_sms, void *stream)
+int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side, void *stream)
 {
     TreeArgs A;
     A.g = args;
@@ -339,10 +372,10 @@ int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side,
     A.g.ntiles = A.g.tiles_x * ((args.ny + side - 1) / side);
     cudaStream_t s = (cudaStream_t)stream;
     switch (op) {
-    case OP_GRAD: return launch_tree_op<OP_GRAD>(A, num_sms, s);
-    case OP_POT: return launch_tree_op<OP_POT>(A, num_sms, s);
-    case OP_HESS: return launch_tree_op<OP_HESS>(A, num_sms, s);
-    case OP_HESS | OP_POT: return launch_tree_op<OP_HESS | OP_POT>(A, num_sms, s);
+    case OP_GRAD: return launch_tree_op<OP_GRAD>(A, s);
+    case OP_POT: return launch_tree_op<OP_POT>(A, s);
+    case OP_HESS: return launch_tree_op<OP_HESS>(A, s);
+    case OP_HESS | OP_POT: return launch_tree_op<OP_HESS | OP_POT>(A, s);
     default: return (int)cudaErrorInvalidValue;
     }
 }
