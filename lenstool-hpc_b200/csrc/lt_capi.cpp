@@ -558,12 +558,12 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
     /* Host outputs: the grid in bands of rows, each band's planes copied to the host on a
      * second stream while the next bands compute.  Every band is launched before the first
      * copy is issued, since a copy into pageable memory returns only once it is done.
-     * Bands start on multiples of the kernels' tile height (8 rows, or the tile side of the
+     * Bands start on multiples of the kernels' tile height (8 rows, or two tiles of the
      * interpolated sums), so every tile covers the pixels it covers in one launch over the
      * whole grid and the maps are the same bit for bit. */
     int band = (int)(((long)g->ny + kHostBands - 1) / kHostBands);
     if (band < kMinBandRows) band = kMinBandRows;
-    const int tile_rows = side ? side : 8;
+    const int tile_rows = side ? 2 * side : 8;
     band = (band + tile_rows - 1) / tile_rows * tile_rows;
     if (!ctx->copy_stream) {
         cudaError_t e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);

@@ -4,9 +4,12 @@
  * Every sum of lt_closed64.cuh is analytic away from its halo, so over a tile of T x T pixels
  * the summed contribution of the halos that are far from the tile is a smooth function: it is
  * evaluated at 16 x 16 Chebyshev nodes of the tile and interpolated to the pixels by the tensor
- * Lagrange polynomial.  Only the halos near the tile are evaluated at its pixels.  A tile then
- * costs 256 (halos) + T^2 (near halos) pairs instead of T^2 (halos).  No counterpart in the
- * reference, which evaluates every pair (src/grid_gradient_GPU.cu:77-179).
+ * Lagrange polynomial; only the halos near the tile are evaluated at its pixels.  The halos that
+ * are far from the square of 2 x 2 tiles around it (its parent) as well are summed at the
+ * parent's nodes instead, once for the four tiles, and interpolated to theirs.  A tile then costs
+ * 64 (halos far from the parent) + 256 (far from the tile only) + T^2 (near halos) pairs instead
+ * of T^2 (halos).  No counterpart in the reference, which evaluates every pair
+ * (src/grid_gradient_GPU.cu:77-179).
  *
  * Which halos are far.  Continued to complex x (or y), a halo's sums are singular where
  * psi = sqrt(q^2 (s^2 + u^2) + v^2) vanishes: at an imaginary distance of at least
@@ -20,19 +23,24 @@
  * shear 3e-15 at 4.0.  A far term is ~1% of its sum, so the truncation stays below the sum's own
  * rounding.
  *
- * Layout.  One CTA of 256 threads a tile: each thread owns one node while the catalogue streams
- * through shared memory (cp.async.bulk, two 64-record stages), then two pixels a pass while the
- * near records, gathered in shared memory, are walked.  Between them the node values are
- * contracted along y for the rows of a pass and along x for each pixel: 17 FP64 operations a
- * pixel and plane.  A tile's time is a latency chain (8 warps, one node a thread), so far records
- * go two at a time: 410 -> 360 us for the deflection of 200 halos on 1024^2 with the rows of
- * tiles launched from the middle outwards, where most halos are, one CTA each (tiles strided over
- * resident CTAs left SMs idle for 26% of the time).
+ * Layout.  One CTA of 256 threads a tile, a cluster of four CTAs a parent.  A CTA sorts the
+ * halos into lists, a halo a thread: its quarter of those far from the parent, those far from its
+ * tile only, those near it; the listed records are gathered in shared memory, 128 at a time, and
+ * each thread sums them at one node of the parent, then of the tile, two records at a time.  The
+ * four shares of the parent's node values are read from the cluster's shared memory and
+ * interpolated to the tile's nodes, those along y to the rows of a pass and along x to each pixel
+ * (17 FP64 operations a pixel and plane); then each thread walks the near records for two pixels.
+ * Bound by the FP64 pipe and, with few tiles, by the dearest tile's chain, so rows of parents
+ * start from the middle of the grid outwards, where most halos are.
+ * B200, ms, tiles alone (no parent, tiles streamed in order) / middle first and two records at a
+ * time / parents: deflection of 200 halos on 1024^2 0.375 / 0.340 / 0.223, of 1000 on 4096^2
+ * 6.6 / 5.03 / 3.27; potential of 200 on 512^2 0.24 / 0.25 / 0.18; lens maps of 500 on 1199 x 901
+ * 1.69 / 1.56 / 1.01.
  */
+#include <algorithm>
 #include <cmath>
 #include <cuda_runtime.h>
 
-#include "lt_bulk.cuh"
 #include "lt_eval.cuh"
 #include "lt_internal.h"
 
@@ -40,37 +48,47 @@ namespace lt {
 
 constexpr int kTreeThreads = 256;
 constexpr int kNodes = 16;
-constexpr int kNearStage = 128; /* near records staged at once: both stages of the walk */
+constexpr int kStage = 128;  /* records staged at once */
+constexpr int kRound = 1024; /* halos classified between two walks */
 constexpr int kNearBlock = 8;
 constexpr int kNearList = 2048; /* near halos of a tile; a tile with more evaluates every halo */
 
-/* Tile sides, and per side the Lagrange basis L[i][c] of the nodes at pixel c of T. */
-constexpr int kSides[] = {32, 48, 64, 128};
-constexpr int kSideTotal = 32 + 48 + 64 + 128;
+/* Tile sides, and per side T the Lagrange basis of the nodes: L[i][c] at pixel c of the tile, and
+ * B[o][i][k] of the parent's nodes at node k of its child o. */
+constexpr int kSides[] = {16, 32, 40, 48, 64, 96, 128};
+constexpr int kSideCount = sizeof(kSides) / sizeof(int);
+constexpr int kSideTotal = 16 + 32 + 40 + 48 + 64 + 96 + 128;
 __device__ double g_nodes[kNodes];
 __device__ double g_lagrange[kNodes * kSideTotal];
+__device__ double g_parent[kSideCount * 2 * kNodes * kNodes];
+
+/* The Lagrange polynomial of node i at x. */
+static double basis(const double *nodes, int i, long double x)
+{
+    long double l = 1.0L;
+    for (int j = 0; j < kNodes; j++)
+        if (j != i) l *= (x - nodes[j]) / ((long double)nodes[i] - nodes[j]);
+    return (double)l;
+}
 
 /* Fill the tables of the current device (identical values every time). */
 int tree_tables()
 {
-    static double nodes[kNodes], lag[kNodes * kSideTotal];
+    static double nodes[kNodes], lag[kNodes * kSideTotal], par[kSideCount * 2 * kNodes * kNodes];
     const long double pi = acosl(-1.0L);
     for (int k = 0; k < kNodes; k++) nodes[k] = (double)cosl((2 * k + 1) * pi / (2 * kNodes));
-    int off = 0;
+    double *l = lag, *p = par;
     for (int T : kSides) {
-        for (int c = 0; c < T; c++) {
-            const long double x = -1.0L + 2.0L * c / (T - 1);
-            for (int i = 0; i < kNodes; i++) {
-                long double l = 1.0L;
-                for (int j = 0; j < kNodes; j++)
-                    if (j != i) l *= (x - nodes[j]) / ((long double)nodes[i] - nodes[j]);
-                lag[off + i * T + c] = (double)l;
-            }
-        }
-        off += kNodes * T;
+        for (int i = 0; i < kNodes; i++)
+            for (int c = 0; c < T; c++) *l++ = basis(nodes, i, -1.0L + 2.0L * c / (T - 1));
+        for (int o = 0; o < 2; o++)
+            for (int i = 0; i < kNodes; i++)
+                for (int k = 0; k < kNodes; k++) /* pixel o T + (T - 1) (1 + node) / 2 of 2 T */
+                    *p++ = basis(nodes, i, -1.0L + 2.0L * (o * T + 0.5L * (T - 1) * (1.0L + nodes[k])) / (2 * T - 1));
     }
     cudaError_t e = cudaMemcpyToSymbol(g_nodes, nodes, sizeof(nodes));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_lagrange, lag, sizeof(lag));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_parent, par, sizeof(par));
     return (int)e;
 }
 
@@ -80,7 +98,20 @@ struct TreeArgs {
     int32_t nhalos;
     int32_t T;            /* tile side */
     int32_t table;        /* its Lagrange table in g_lagrange */
+    int32_t parent;       /* and in g_parent */
 };
+
+/* The cluster's barrier, and a double of CTA `rank`'s shared memory. */
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ double cluster_load(const double *p, int rank)
+{
+    uint32_t addr = (uint32_t)__cvta_generic_to_shared(p), at;
+    double v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
+    return v;
+}
 
 template <int OP>
 struct TreeOp {
@@ -88,13 +119,14 @@ struct TreeOp {
     static constexpr double far = OP & OP_HESS ? 4.0 : OP & OP_GRAD ? 3.2 : 3.0;
 };
 
-/* Shared memory: the two stages, node values, one pass's row values, the Lagrange table. */
+/* Shared memory: the stage, node values of the tile and of this CTA's share of the parent's, one
+ * pass's row values, the Lagrange table, the lists. */
 template <int OP>
 static size_t tree_smem(int T)
 {
-    return 2 * LT_CHUNK * sizeof(lt_nie64) +
-           sizeof(double) * (TreeOp<OP>::planes * kNodes * (kNodes + 2 * kTreeThreads / T) + kNodes * T) +
-           sizeof(int32_t) * kNearList;
+    return kStage * sizeof(lt_nie64) +
+           sizeof(double) * (TreeOp<OP>::planes * kNodes * (2 * kNodes + 2 * kTreeThreads / T) + kNodes * T) +
+           sizeof(int32_t) * (kNearList + kRound + kRound / 4);
 }
 
 template <int OP, int TYPE, int P>
@@ -152,112 +184,16 @@ __device__ __forceinline__ void tree_two(int type, const lt_nie64 &r0, const lt_
     for (int q = 0; q < TreeOp<OP>::planes; q++) s[0][q] += t[0][0][q] + t[1][0][q];
 }
 
+/* The pixels of a tile: the interpolated far sums and its near halos, two pixels a thread a pass. */
 template <int OP>
-__global__ void __launch_bounds__(kTreeThreads, 2) tree64_kernel(const TreeArgs A)
+__device__ __forceinline__ void tree_pixels(const TreeArgs &A, unsigned char *smem, int32_t *s_type,
+                                            const int32_t *list, int near, int tx0, int ty0, const double *F, double *H,
+                                            const double *L)
 {
     constexpr int NQ = TreeOp<OP>::planes;
     const GridArgs &a = A.g;
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ __align__(8) uint64_t bars[2];
-    __shared__ uint32_t s_far[2];
-    __shared__ int32_t s_type[kNearStage];
-    __shared__ int s_near;
     lt_nie64 *stage = reinterpret_cast<lt_nie64 *>(smem);
-    const int T = A.T, rows = 2 * kTreeThreads / T;
-    double *F = reinterpret_cast<double *>(smem + 2 * LT_CHUNK * sizeof(lt_nie64)); /* [plane][j][i] */
-    double *H = F + NQ * kNodes * kNodes;                                           /* [plane][row][i] */
-    double *L = H + NQ * kNodes * rows;                                             /* [i][column] */
-    int32_t *list = reinterpret_cast<int32_t *>(L + kNodes * T);
-
-    const int tid = threadIdx.x;
-    if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        mbar_fence_init();
-    }
-    for (int e = tid; e < kNodes * T; e += kTreeThreads) L[e] = g_lagrange[A.table + e];
-    const double node_x = g_nodes[tid & 15], node_y = g_nodes[tid >> 4];
-    uint32_t phase[2] = {0, 0};
-    __syncthreads();
-
-    auto issue = [&](int ci) {
-        const lt_chunk c = a.chunks[ci];
-        fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&bars[ci & 1], (uint32_t)c.count * (uint32_t)sizeof(lt_nie64));
-        bulk_g2s(stage + (ci & 1) * LT_CHUNK, a.nie + c.start, (uint32_t)c.count * (uint32_t)sizeof(lt_nie64),
-                 &bars[ci & 1]);
-    };
-
-    /* rows of tiles from the middle outwards: the halos crowd there, and the dear tiles go first */
-    const int trows = a.ntiles / a.tiles_x, mid = (trows - 1) / 2;
-    const int r = (int)blockIdx.x / a.tiles_x, row = mid + ((r & 1) ? (r + 1) / 2 : -(r / 2));
-    const int tx0 = ((int)blockIdx.x % a.tiles_x) * T, ty0 = row * T;
-    const double x0 = pixel_x(a, tx0), x1 = pixel_x(a, tx0 + T - 1);
-    const double y0 = pixel_y(a, ty0), y1 = pixel_y(a, ty0 + T - 1);
-    const double xc = 0.5 * (x0 + x1), yc = 0.5 * (y0 + y1), hx = 0.5 * (x1 - x0), hy = 0.5 * (y1 - y0);
-    const double diag = sqrt(hx * hx + hy * hy), reach = TreeOp<OP>::far * fmax(fabs(hx), fabs(hy));
-
-    /* the walk: near halos to the list, far ones summed at this thread's node */
-    double f[1][NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) f[0][q] = 0.;
-    const double nx[1] = {fma(hx, node_x, xc)}, ny[1] = {fma(hy, node_y, yc)};
-    int nlist = 0; /* warp 0's count of near halos */
-    if (tid == 0) issue(0);
-    for (int ci = 0; ci < a.nchunks; ci++) {
-        const int b = ci & 1;
-        if (tid == 0 && ci + 1 < a.nchunks) issue(ci + 1);
-        if (!wait_tile(&bars[b], phase[b], a.status)) {
-            if (tid == 0 && ci + 1 < a.nchunks) drain_tile(&bars[b ^ 1], phase[b ^ 1]);
-            return;
-        }
-        phase[b] ^= 1;
-        const lt_chunk c = a.chunks[ci];
-        const lt_nie64 *recs = stage + b * LT_CHUNK;
-        if (tid < 32) { /* one warp, so that the list keeps the catalogue's order */
-#pragma unroll
-            for (int w = 0; w < 2; w++) {
-                const int i = 32 * w + tid;
-                bool far = false;
-                if (i < c.count) {
-                    const lt_nie64 &r = recs[i];
-                    const double dx = r.x0 - xc, dy = r.y0 - yc;
-                    const double d = fmax(sqrt(dx * dx + dy * dy) - diag, 0.);
-                    const double s = c.type == 5 ? 0. : r.sc;
-                    far = (c.type == 5 ? r.q2 / r.k : r.q2) * (d * d + s * s) >= reach * reach;
-                }
-                const uint32_t m = __ballot_sync(0xffffffffu, far);
-                const uint32_t near = __ballot_sync(0xffffffffu, i < c.count && !far);
-                const int at = nlist + __popc(near & ((1u << tid) - 1u));
-                if (i < c.count && !far && at < kNearList) list[at] = c.start + i;
-                nlist += __popc(near);
-                if (tid == 0) s_far[w] = m;
-            }
-        }
-        __syncthreads();
-        double fc[1][NQ]; /* the chunk's own sum: fewer roundings of the large total */
-#pragma unroll
-        for (int q = 0; q < NQ; q++) fc[0][q] = 0.;
-#pragma unroll 1
-        for (uint64_t m = (uint64_t)s_far[1] << 32 | s_far[0]; m;) { /* two records at a time */
-            const int i = __ffsll(m) - 1;
-            m &= m - 1;
-            const int j = m ? __ffsll(m) - 1 : -1;
-            m &= m - 1;
-            if (j >= 0)
-                tree_two<OP>(c.type, recs[i], recs[j], nx, ny, a.kmap, fc);
-            else
-                tree_any<OP, 1>(c.type, recs[i], nx, ny, a.kmap, fc);
-        }
-#pragma unroll
-        for (int q = 0; q < NQ; q++) f[0][q] += fc[0][q];
-        __syncthreads(); /* the stage and s_far are refilled */
-    }
-#pragma unroll
-    for (int q = 0; q < NQ; q++) F[q * kNodes * kNodes + tid] = f[0][q];
-    if (tid == 0) s_near = nlist;
-    __syncthreads();
-    int near = s_near;
+    const int T = A.T, rows = 2 * kTreeThreads / T, tid = threadIdx.x;
     const bool all = near > kNearList; /* more than the list holds: every halo at every pixel */
     if (all) near = A.nhalos;
     auto gather = [&](int i0, int n) { /* near records i0 .. i0 + n - 1 */
@@ -268,7 +204,7 @@ __global__ void __launch_bounds__(kTreeThreads, 2) tree64_kernel(const TreeArgs 
         }
         for (int e = tid; e < n; e += kTreeThreads) s_type[e] = A.types[all ? i0 + e : list[i0 + e]];
     };
-    if (near <= kNearStage) gather(0, near);
+    if (near <= kStage) gather(0, near);
 
     for (int r0 = 0; r0 < T && ty0 + r0 < a.ny; r0 += rows) {
         __syncthreads(); /* F and the gathered records; H is free */
@@ -295,9 +231,9 @@ __global__ void __launch_bounds__(kTreeThreads, 2) tree64_kernel(const TreeArgs 
 #pragma unroll
             for (int q = 0; q < NQ; q++) s[k][q] = 0.;
         }
-        for (int i0 = 0; i0 < near; i0 += kNearStage) {
-            const int n = near - i0 < kNearStage ? near - i0 : kNearStage;
-            if (near > kNearStage) {
+        for (int i0 = 0; i0 < near; i0 += kStage) {
+            const int n = near - i0 < kStage ? near - i0 : kStage;
+            if (near > kStage) {
                 __syncthreads();
                 gather(i0, n);
                 __syncthreads();
@@ -347,11 +283,191 @@ __global__ void __launch_bounds__(kTreeThreads, 2) tree64_kernel(const TreeArgs 
     }
 }
 
+/* Records [b, e) of the stage summed at one node a thread, two at a time where they are alike. */
+template <int OP>
+__device__ __forceinline__ void tree_walk(const lt_nie64 *stage, const int32_t *type, int b, int e,
+                                          const double (&px)[1], const double (&py)[1], int kmap, double *out)
+{
+    constexpr int NQ = TreeOp<OP>::planes;
+    if (b >= e) return;
+    double fc[1][NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) fc[0][q] = 0.;
+#pragma unroll 1
+    for (; b < e; b++) {
+        if (b + 1 < e && type[b] == type[b + 1]) {
+            tree_two<OP>(type[b], stage[b], stage[b + 1], px, py, kmap, fc);
+            b++;
+        } else
+            tree_any<OP, 1>(type[b], stage[b], px, py, kmap, fc);
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; q++) out[q * kNodes * kNodes] += fc[0][q];
+}
+
+/* The centre, half widths and reach of a square of tiles. */
+struct Square {
+    double xc, yc, hx, hy, diag, reach2;
+    __device__ __forceinline__ Square(const GridArgs &a, int tx0, int ty0, int T, double far)
+    {
+        const double x0 = pixel_x(a, tx0), x1 = pixel_x(a, tx0 + T - 1);
+        const double y0 = pixel_y(a, ty0), y1 = pixel_y(a, ty0 + T - 1);
+        xc = 0.5 * (x0 + x1);
+        yc = 0.5 * (y0 + y1);
+        hx = 0.5 * (x1 - x0);
+        hy = 0.5 * (y1 - y0);
+        diag = sqrt(hx * hx + hy * hy);
+        const double r = far * fmax(fabs(hx), fabs(hy));
+        reach2 = r * r;
+    }
+    __device__ __forceinline__ bool is_far(double x, double y, double q2, double s2) const
+    {
+        const double dx = x - xc, dy = y - yc, d = fmax(sqrt(dx * dx + dy * dy) - diag, 0.);
+        return q2 * (d * d + s2) >= reach2;
+    }
+};
+
+template <int OP>
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kTreeThreads, 2) tree64_kernel(const TreeArgs A)
+{
+    constexpr int NQ = TreeOp<OP>::planes, NN = kNodes * kNodes;
+    const GridArgs &a = A.g;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int32_t s_type[kStage];
+    __shared__ int s_cnt[2][3][kTreeThreads / 32];
+    lt_nie64 *stage = reinterpret_cast<lt_nie64 *>(smem);
+    const int T = A.T, rows = 2 * kTreeThreads / T;
+    double *F = reinterpret_cast<double *>(smem + kStage * sizeof(lt_nie64)); /* [plane][j][i] */
+    double *S = F + NQ * NN;                                                  /* the share, [plane][j][i] */
+    double *H = S + NQ * NN;                                                  /* [plane][row][i] */
+    double *L = H + NQ * kNodes * rows;                                       /* [i][column] */
+    int32_t *list = reinterpret_cast<int32_t *>(L + kNodes * T);              /* near halos */
+    int32_t *own = list + kNearList, *share = own + kRound;                   /* far halos of a round */
+
+    const int tid = threadIdx.x, rank = blockIdx.x & 3;
+    for (int e = tid; e < kNodes * T; e += kTreeThreads) L[e] = g_lagrange[A.table + e];
+    const double node_x = g_nodes[tid & 15], node_y = g_nodes[tid >> 4];
+
+    /* rows of clusters from the middle outwards: the halos crowd there, and the dear tiles go first */
+    const int ccols = (a.tiles_x + 1) / 2, crows = (int)gridDim.x / (4 * ccols), cl = (int)blockIdx.x >> 2;
+    const int r = cl / ccols, crow = (crows - 1) / 2 + ((r & 1) ? (r + 1) / 2 : -(r / 2));
+    const int px0 = 2 * T * (cl % ccols), py0 = 2 * T * crow;
+    const int tx0 = px0 + (rank & 1) * T, ty0 = py0 + (rank >> 1) * T;
+    const bool alive = tx0 < a.nx && ty0 < a.ny; /* a tile beyond the grid does its share only */
+    const Square P(a, px0, py0, 2 * T, TreeOp<OP>::far), C(a, tx0, ty0, T, TreeOp<OP>::far);
+
+#pragma unroll
+    for (int q = 0; q < NQ; q++) F[q * NN + tid] = S[q * NN + tid] = 0.;
+    int near = 0;
+    for (int base = 0; base < A.nhalos; base += kRound) {
+        /* the round's halos to the lists, in the catalogue's order: far from the parent (this
+         * CTA's quarter of them), far from the tile only, near */
+        int nshare = 0, nown = 0;
+        for (int sub = 0; sub < kRound && base + sub < A.nhalos; sub += kTreeThreads) {
+            const int i = base + sub + tid;
+            int cls = -1;
+            if (i < A.nhalos) {
+                const lt_nie64 &h = a.nie[i];
+                const bool point = A.types[i] == 5;
+                const double x = h.x0, y = h.y0, q2 = point ? h.q2 / h.k : h.q2, s = point ? 0. : h.sc;
+                if (P.is_far(x, y, q2, s * s))
+                    cls = (i & 3) == rank ? 0 : -1;
+                else if (alive)
+                    cls = C.is_far(x, y, q2, s * s) ? 1 : 2;
+            }
+            int at[3], tot[3];
+            int (*cnt)[kTreeThreads / 32] = s_cnt[(sub / kTreeThreads) & 1];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const uint32_t m = __ballot_sync(0xffffffffu, cls == k);
+                at[k] = __popc(m & ((1u << (tid & 31)) - 1u));
+                if ((tid & 31) == 0) cnt[k][tid >> 5] = __popc(m);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                tot[k] = 0;
+#pragma unroll
+                for (int w = 0; w < kTreeThreads / 32; w++) {
+                    if (w == tid >> 5) at[k] += tot[k];
+                    tot[k] += cnt[k][w];
+                }
+            }
+            if (cls == 0) share[nshare + at[0]] = i;
+            if (cls == 1) own[nown + at[1]] = i;
+            if (cls == 2 && near + at[2] < kNearList) list[near + at[2]] = i;
+            nshare += tot[0];
+            nown += tot[1];
+            near += tot[2];
+        }
+        /* their sums at this thread's node of the parent and of the tile */
+        const int nfar = nshare + nown;
+        for (int b = 0; b < nfar; b += kStage) {
+            const int n = nfar - b < kStage ? nfar - b : kStage;
+            __syncthreads(); /* the lists; the stage is free */
+            for (int e = tid; e < n * (int)(sizeof(lt_nie64) / 16); e += kTreeThreads) {
+                const int k = b + e / (int)(sizeof(lt_nie64) / 16);
+                const int4 *src = reinterpret_cast<const int4 *>(a.nie + (k < nshare ? share[k] : own[k - nshare]));
+                reinterpret_cast<int4 *>(stage)[e] = src[e % (int)(sizeof(lt_nie64) / 16)];
+            }
+            for (int e = tid; e < n; e += kTreeThreads)
+                s_type[e] = A.types[b + e < nshare ? share[b + e] : own[b + e - nshare]];
+            __syncthreads();
+            const int m = nshare - b < 0 ? 0 : nshare - b < n ? nshare - b : n;
+#pragma unroll 1
+            for (int k = 0; k < 2; k++) {
+                const double nx[1] = {k ? fma(C.hx, node_x, C.xc) : fma(P.hx, node_x, P.xc)};
+                const double ny[1] = {k ? fma(C.hy, node_y, C.yc) : fma(P.hy, node_y, P.yc)};
+                tree_walk<OP>(stage, s_type, k ? m : 0, k ? n : m, nx, ny, a.kmap, (k ? F : S) + tid);
+            }
+        }
+        __syncthreads(); /* the lists are refilled */
+    }
+
+    /* the parent's node values, summed over the cluster, interpolated to the tile's nodes */
+    cluster_arrive();
+    cluster_wait();
+    double *PP = reinterpret_cast<double *>(stage), *G = PP + NQ * NN; /* [plane][j][i] */
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+        double v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = cluster_load(S + q * NN + tid, k);
+        PP[q * NN + tid] = (v[0] + v[1]) + (v[2] + v[3]);
+    }
+    cluster_arrive(); /* the shares are read: waited for before the exit */
+    if (alive) {
+        __syncthreads();
+        const double *bx = g_parent + A.parent + (rank & 1) * NN, *by = g_parent + A.parent + (rank >> 1) * NN;
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            double g = 0.;
+#pragma unroll
+            for (int i = 0; i < kNodes; i++)
+                g = fma(bx[i * kNodes + (tid & 15)], PP[q * NN + (tid & ~15) + i], g);
+            G[q * NN + tid] = g;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            double g = 0.;
+#pragma unroll
+            for (int j = 0; j < kNodes; j++)
+                g = fma(by[j * kNodes + (tid >> 4)], G[q * NN + j * kNodes + (tid & 15)], g);
+            F[q * NN + tid] += g;
+        }
+        __syncthreads(); /* F; the stage is free */
+        tree_pixels<OP>(A, smem, s_type, list, near, tx0, ty0, F, H, L);
+    }
+    cluster_wait();
+}
+
 template <int OP>
 static int launch_tree_op(TreeArgs &A, cudaStream_t s)
 {
     const size_t smem = tree_smem<OP>(A.T);
-    tree64_kernel<OP><<<A.g.ntiles, kTreeThreads, smem, s>>>(A);
+    const int clusters = ((A.g.tiles_x + 1) / 2) * ((A.g.ntiles / A.g.tiles_x + 1) / 2);
+    tree64_kernel<OP><<<4 * clusters, kTreeThreads, smem, s>>>(A);
     count_launch(1);
     return (int)cudaGetLastError();
 }
@@ -363,10 +479,11 @@ int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side,
     A.types = reinterpret_cast<const Fp32cCatalog *>(&cat->aux_desc)->types;
     A.nhalos = cat->nhalos;
     A.T = side;
-    A.table = 0;
+    A.table = A.parent = 0;
     for (int T : kSides) {
         if (T == side) break;
         A.table += kNodes * T;
+        A.parent += 2 * kNodes * kNodes;
     }
     A.g.tiles_x = (args.nx + side - 1) / side;
     A.g.ntiles = A.g.tiles_x * ((args.ny + side - 1) / side);
@@ -381,14 +498,17 @@ int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side,
 }
 
 /* The tile side for sums `op` of a grid, or 0 where the direct kernels are the faster: costs in
- * pairs per resident CTA (two an SM).  A tile costs 256 halos at the nodes (one pair a thread
- * in flight there instead of two, and the walk's barriers: x 1.25) and its near halos at T^2
- * pixels; the halos count as spread over their bounding box, tiles inside it being the dearest.
- * B200, ms, every pair / sides 32, 48, 64, 128: deflection of 200 halos on 1024^2 1.41 / 0.51,
- * 0.40, 0.38, 2.58; of 1000 on 4096^2 110 / 31.3, 14.7, 8.8, 6.6; of 1000 on 500^2 2.00 / 0.77,
- * 1.37, 3.14, 23; potential of 1000 on 2048^2 45.3 / 11.6, 6.0, 4.3, 10.2; lens maps of 500 on
- * 1199 x 901 7.11 / 2.18, 1.72, 1.74, 13.2.  The rule takes 0.41, 6.8, 0.78, 4.3 and 1.69
- * (block sums included). */
+ * pairs per resident CTA (two an SM), fitted to 54 measured combinations of sum, grid (96^2 to
+ * 4096^2) and halos (10 to 1000).  A tile costs its lists and quarter of the parent's nodes (57 a
+ * halo: 64 pairs, cheaper for the halos that are not far), its own nodes for the halos that are
+ * near the parent only, its passes of 512 pixels with the near halos and the interpolation; the
+ * halos count as spread over their bounding box, tiles inside it being the dearest, and such a
+ * tile alone on its SM runs at twice the rate.  The direct kernels cost their waves and the chain
+ * of one record after another.  B200, ms, every pair / sides 16, 32, 40, 48, 64, 128, the pick in
+ * brackets: deflection of 200 halos on 256^2 0.14 / [0.07] 0.14 0.28 0.43; of 1000 on 500^2
+ * 2.00 / - [0.53] 1.00 1.43 3.2 23; of 200 on 1024^2 1.41 / - [0.22] 0.23 0.24 0.35 2.5; of 350 on
+ * 1501 x 777 2.14 / - 0.32 [0.30] 0.33 0.42 2.7; of 1000 on 4096^2 110 / - 8.7 6.3 4.7 [3.3] 4.5;
+ * lens maps of 300 on 96^2 [0.12] / 0.32 0.72. */
 int tree_side(const lt_catalog *cat, int op, int nx, int ny, double dx, double dy, int num_sms)
 {
     const double n = cat->nhalos, slots = 2. * num_sms;
@@ -397,16 +517,18 @@ int tree_side(const lt_catalog *cat, int op, int nx, int ny, double dx, double d
     const double spread = M_PI * (far * far * cat->sum_iq2 + 2. * d * far * cat->sum_iq + 2. * n);
     const double grid = std::fabs(nx * dx * ny * dy), box = cat->box;
     const double pixels = (double)nx * ny;
-    double best = 0.8 * n * 512. * std::ceil(pixels / (512. * slots));
+    double best = 512. * n * (0.265 + pixels / (512. * slots));
     int side = 0;
     for (int T : kSides) {
         const double h = 0.5 * T * std::fmax(std::fabs(dx), std::fabs(dy));
-        const double tiles = std::ceil(nx / (double)T) * std::ceil(ny / (double)T);
+        const double tiles = 4. * std::ceil(nx / (2. * T)) * std::ceil(ny / (2. * T));
+        const int rows = 2 * kTreeThreads / T, passes = (T + rows - 1) / rows;
         auto cost = [&](double area) {
             const double near = area > 0. ? std::fmin(n, h * h * spread / area) : n;
-            return 320. * n + (double)T * T * (1.1 * near + 1.5) + 4000.;
+            const double parent = std::fmin(n, 4. * near);
+            return 57. * n + 310. * (parent - near) + 512. * passes * (1.22 * near + 4.9) + 3250.;
         };
-        const double t = std::fmax(tiles * cost(std::fmax(grid, box)) / slots, cost(std::fmin(grid, box)));
+        const double t = std::fmax(tiles * cost(std::fmax(grid, box)) / slots, 0.5 * cost(std::fmin(grid, box)));
         if (t < best) {
             best = t;
             side = T;
@@ -418,7 +540,9 @@ int tree_side(const lt_catalog *cat, int op, int nx, int ny, double dx, double d
 template <int OP>
 static cudaError_t allow_smem()
 {
-    return cudaFuncSetAttribute(tree64_kernel<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tree_smem<OP>(128) + 4096);
+    size_t most = 0;
+    for (int T : kSides) most = std::max(most, tree_smem<OP>(T));
+    return cudaFuncSetAttribute(tree64_kernel<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
 /* Once per context: the kernels' shared memory on the current device. */

@@ -58,6 +58,8 @@ GRIDS = {
     "falling": catalog.Grid(100., -100., 60., -90., 600, 450, dx=-200. / 599, dy=-150. / 449),
     "offset": catalog.Grid(-200., 200., -150., 150., 617, 401, 333, 250, dx=0.21, dy=0.34),
     "cut-out": catalog.Grid(5., 35., -40., -10., 512, 512),
+    "small": catalog.Grid.square(100., 250),
+    "one parent wide": catalog.Grid(-3., 3., -90., 90., 50, 3000),
 }
 
 
