@@ -184,6 +184,7 @@ lt_status lt_batch_create(lt_context *ctx, const lt_request *reqs, int32_t nreqs
         q.state = b->state;
         q.nslots = nreqs;
         q.window = 1;
+        q.refilled = 0;
         q.idle_polls = 0;
         q.desc_polls = 1 << 30; /* every descriptor is in place before the graph runs */
         q.status = ctx->status;

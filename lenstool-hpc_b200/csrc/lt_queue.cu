@@ -344,7 +344,7 @@ __device__ int claim_tile(const QArgs &q, int &slot_out, int &tile_out, uint32_t
         if (h >= p) return 0;
         unsigned long long span = p - h;
         if (span > (unsigned long long)q.window) span = (unsigned long long)q.window;
-        const unsigned long long r0 = atomicAdd(&st->rotor, 1ull);
+        const unsigned long long r0 = span > 1 ? atomicAdd(&st->rotor, 1ull) : 0ull;
         bool head_exhausted = false, head_missing = false;
         for (unsigned long long k = 0; k < span; k++) {
             const unsigned long long r = h + (r0 + k) % span;
@@ -353,10 +353,13 @@ __device__ int claim_tile(const QArgs &q, int &slot_out, int &tile_out, uint32_t
             const int nt = __ldcg(&s->item.ntiles);
             const uint32_t seq = (uint32_t)__ldcg(reinterpret_cast<const int *>(&s->item.seq));
             while ((uint32_t)(c >> 32) == (uint32_t)r && seq == (uint32_t)r && (int)(c & 0xffffffffu) < nt) {
-                const unsigned long long prev = atomicCAS(&s->ctr, c, c + 1ull);
-                if (prev == c) {
+                /* a slot that is not refilled is counted up past its last tile, by at most
+                 * one for each CTA; in one that is, an addition could land on the request
+                 * after r, so the claim has to compare */
+                const unsigned long long prev = q.refilled ? atomicCAS(&s->ctr, c, c + 1ull) : atomicAdd(&s->ctr, 1ull);
+                if (q.refilled ? prev == c : (int)(prev & 0xffffffffu) < nt) {
                     slot_out = (int)(r % (unsigned long long)q.nslots);
-                    tile_out = (int)(c & 0xffffffffu);
+                    tile_out = (int)(prev & 0xffffffffu);
                     return 1;
                 }
                 c = prev;

@@ -57,6 +57,7 @@ struct QArgs {
     QState *state;
     int32_t nslots;
     int32_t window;                /* requests served round-robin (1: first come, first served) */
+    int32_t refilled;              /* slots take later requests while the kernel runs        */
     int32_t idle_polls;            /* polls of ~1 us before an idle CTA leaves */
     int32_t desc_polls;            /* polls of ~1 us a CTA waits for the descriptor of the oldest
                                       published request before reporting LT_ERR_TIMEOUT */

@@ -412,6 +412,7 @@ void keep_loop(lt_server *s)
     q.state = s->state;
     q.nslots = s->nslots;
     q.window = s->window;
+    q.refilled = 1;
     q.idle_polls = s->idle_polls;
     q.desc_polls = s->desc_polls;
     q.status = s->ctx->status;
