@@ -50,6 +50,7 @@
 namespace lt {
 
 constexpr int kQThreads = 256;
+constexpr int kListed = 2 * kQThreads; /* a tile's pixels at most, two a thread */
 
 /* ------------------------------------------------------------------ device ---- */
 
@@ -189,11 +190,10 @@ __device__ __noinline__ bool tile64(const QItem &it, int tile, Stage &st, int32_
 }
 
 /* FP32C (or, with an all-FP64 chunk list, fast FP64) Hessian/potential sums of one tile:
- * grid32c_kernel's per-tile work followed by the FP64 recomputation of the tile's
- * pixels whose FP32 error bound on mu exceeds mu_tol (the single-grid path's second pass,
- * same arithmetic). */
+ * grid32c_kernel's per-tile work; the pixels whose FP32 error bound on mu exceeds mu_tol are
+ * added to the CTA's list. */
 template <int OP, int P>
-__device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_t *status, int16_t *s_list, int *s_count)
+__device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_t *status, int2 *s_list, int *s_count)
 {
     const GridArgs &a = it.g;
     int ix, iy;
@@ -232,8 +232,6 @@ __device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_
                           });
     if (!ok) return false;
     const bool recompute = (OP & OP_HESS) && it.mu_tol > 0.;
-    if (recompute && threadIdx.x == 0) *s_count = 0;
-    if (recompute) __syncthreads();
     if (iy < a.ny) {
         const long row = (long)iy * a.nx;
         double hxx[P], hyy[P], hxy[P], psi[P], gx[P], gy[P];
@@ -262,25 +260,21 @@ __device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_
                     if (ix + k < a.nx) dst[k] = v[k];
             }
         }
-        if (recompute) {
-            const int tile_x0 = (tile % a.tiles_x) * 32 * P, tile_y0 = (tile / a.tiles_x) * 8;
 #pragma unroll
-            for (int k = 0; k < P; k++)
-                if (flag[k] && ix + k < a.nx) {
-                    const int slot = atomicAdd(s_count, 1);
-                    s_list[slot] = (int16_t)((iy - tile_y0) * 32 * P + (ix + k - tile_x0));
-                }
-        }
+        for (int k = 0; k < P; k++)
+            if (flag[k] && ix + k < a.nx) s_list[atomicAdd(s_count, 1)] = make_int2(ix + k, iy);
     }
-    if (!recompute) return true;
-    __syncthreads();
-    /* the flagged pixels (at most the tile's 32 P x 8 = P kQThreads), in one walk of the
-     * catalogue's FP64 closed-form records: thread t takes entries t and t + kQThreads; a warp
-     * with no second entry evaluates one pixel a thread (an empty second pixel would double
-     * its work) */
-    const int n = *s_count;
-    const int tile_x0 = (tile % a.tiles_x) * 32 * P, tile_y0 = (tile / a.tiles_x) * 8;
-    if (n == 0) return true;
+    return true;
+}
+
+/* FP64 recomputation of `n` listed pixels (at most 2 kQThreads; the single-grid path's second
+ * pass, same arithmetic), in one walk of the catalogue's FP64 closed-form records: thread t takes
+ * entries t and t + kQThreads; a warp with no second entry evaluates one pixel a thread (an empty
+ * second pixel would double its work). */
+__device__ __noinline__ bool recompute_listed(const QItem &it, Stage &st, int32_t *status, const int2 *s_list, int n)
+{
+    constexpr int P = 2;
+    const GridArgs &a = it.g;
     /* the count of recomputed pixels (lt_recompute_count): word 2 of the status block */
     if (threadIdx.x == 0 && status)
         atomicAdd(reinterpret_cast<unsigned long long *>(status + 2), (unsigned long long)n);
@@ -291,14 +285,14 @@ __device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_
     for (int k = 0; k < P; k++) {
         const int e = k * kQThreads + (int)threadIdx.x;
         have[k] = e < n;
-        const int l = have[k] ? s_list[e] : 0;
-        qx[k] = tile_x0 + l % (32 * P);
-        qy[k] = tile_y0 + l / (32 * P);
+        const int2 l = have[k] ? s_list[e] : make_int2(0, 0);
+        qx[k] = l.x;
+        qy[k] = l.y;
         qpx[k] = pixel_x(a, qx[k]);
         qpy[k] = pixel_y(a, qy[k]);
         kap[k] = g1[k] = g2[k] = 0.;
     }
-    const bool one = !__any_sync(0xffffffffu, P == 2 && have[P - 1]); /* warp-uniform */
+    const bool one = !__any_sync(0xffffffffu, have[1]); /* warp-uniform */
     double px1[1] = {qpx[0]}, py1[1] = {qpy[0]}, kap1[1] = {0.}, g11[1] = {0.}, g21[1] = {0.};
     const bool ok2 = walk_chunks(st, a.chunks, a.nchunks, static_cast<const lt_rec64 *>(recs_of<OP_NI>(a, 0)), nullptr,
                                  status, [&](const lt_chunk &c, const unsigned char *buf) {
@@ -307,7 +301,7 @@ __device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_
                                      if (one)
                                          eval_nie_chunk<1, 4>(c, recs, px1, py1, a.kmap, kap1, g11, g21);
                                      else
-                                         eval_nie_chunk<P>(c, recs, qpx, qpy, a.kmap, kap, g1, g2);
+                                         eval_nie_chunk<P, 2>(c, recs, qpx, qpy, a.kmap, kap, g1, g2);
                                  });
     if (!ok2) return false;
     if (one) {
@@ -390,7 +384,7 @@ __global__ void __launch_bounds__(kQThreads, MINB) queue_kernel(const QArgs q)
     __shared__ __align__(8) uint64_t bars[2];
     __shared__ __align__(16) QItem item;
     __shared__ int s_slot, s_tile, s_count;
-    __shared__ int16_t s_list[kQThreads * 2];
+    __shared__ int2 s_list[2 * kListed]; /* flagged pixels of request s_slot not yet recomputed */
     const int tid = threadIdx.x;
     Stage st;
     st.buf[0] = smem;
@@ -402,8 +396,19 @@ __global__ void __launch_bounds__(kQThreads, MINB) queue_kernel(const QArgs q)
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         mbar_fence_init();
+        s_count = 0;
     }
     __syncthreads();
+    /* recompute the last of the listed pixels, kListed at most */
+    auto recompute = [&]() -> bool {
+        const int count = s_count, n = count < kListed ? count : kListed;
+        const bool ok = recompute_listed(item, st, q.status, s_list + (count - n), n);
+        __syncthreads();
+        if (tid == 0) s_count = count - n;
+        __syncthreads();
+        return ok;
+    };
+    int current = -1; /* the slot whose item is in shared memory */
     for (;;) {
         if (tid == 0) {
             int slot = -1, tile = 0;
@@ -451,12 +456,14 @@ __global__ void __launch_bounds__(kQThreads, MINB) queue_kernel(const QArgs q)
         }
         __syncthreads();
         const int slot = s_slot, tile = s_tile;
+        if (MODE == QMODE_C32 && slot != current && s_count > 0 && !recompute()) break;
         if (slot < 0) break;
-        {
+        if (slot != current || q.refilled) {
             const int4 *src = reinterpret_cast<const int4 *>(&q.slots[slot].item);
             int4 *dst = reinterpret_cast<int4 *>(&item);
             for (int i = tid; i < (int)(sizeof(QItem) / 16); i += kQThreads) dst[i] = __ldcg(src + i);
         }
+        current = slot;
         __syncthreads();
         bool ok = true;
         if (MODE == QMODE_C32) {
@@ -466,6 +473,11 @@ __global__ void __launch_bounds__(kQThreads, MINB) queue_kernel(const QArgs q)
             if (ok && hp == OP_POT) ok = tile32<OP_POT, P32>(item, tile, st, q.status, s_list, &s_count);
             if (ok && hp == (OP_HESS | OP_POT))
                 ok = tile32<OP_HESS | OP_POT, P32>(item, tile, st, q.status, s_list, &s_count);
+            __syncthreads();
+            /* A batch's flagged pixels wait until each thread has two of them (a tile's own,
+             * half of 512 at 200 halos, leave warps without a pixel); a server's are done with
+             * their tile, which may be the request's last.  */
+            if (ok && s_count >= (q.refilled ? 1 : kListed)) ok = recompute();
         } else {
             if (item.op & OP_GRAD) ok = tile64<OP_GRAD, 2>(item, tile, st, q.status);
             if (ok && (item.op & OP_HESS)) ok = tile64<OP_HEX, 2>(item, tile, st, q.status);
