@@ -275,8 +275,9 @@ lt_status lt_set_kernel_config(lt_context *ctx, int32_t precision, int32_t sums,
 lt_status lt_get_kernel_config(const lt_context *ctx, int32_t precision, int32_t sums, lt_kernel_config *config);
 /* Time every configuration for (precision, sums) on a grid_n x grid_n grid covering the
  * catalogue and keep the fastest in the context; *best_ms (may be NULL) gets its time.
- * The batches built afterwards use the tuned LT_FP32C Hessian shape where their
- * persistent kernel is built for it (pixels per thread and CTAs per SM at 256 threads). */
+ * The batches built afterwards take the pixels per thread of the tuned LT_FP32C Hessian
+ * shape; their persistent kernel has 256 threads and two CTAs per SM (one where the batch
+ * has no more tiles than the GPU SMs). */
 lt_status lt_autotune(lt_context *ctx, const lt_catalog *cat, int32_t precision, int32_t sums, int32_t grid_n,
                       double *best_ms);
 
@@ -299,7 +300,9 @@ lt_status lt_recompute_count(lt_context *ctx, uint64_t *pixels);
  * A request is one grid of output planes over one uploaded catalogue: any mix of Hessian
  * maps (lt_map_kind 0-41, with `dlsds` as D, `kmap` and `mult` as in lt_hessian_maps),
  * the potential and the deflection (both multiplied by `scale`).  Results equal those of
- * the single-grid calls in the same precision (LT_FP32C or LT_FP64) bit for bit.
+ * the single-grid calls in the same precision bit for bit for LT_FP32C and the LT_FP64
+ * Hessian; the LT_FP64 deflection and potential, whose far halos the single-grid calls
+ * interpolate, agree to 1e-13 of max(|value|, RMS).
  * No counterpart in the reference, whose posterior driver makes one blocking map call
  * per sample (utils/maps/main.cpp:432-587). */
 typedef struct {

@@ -135,19 +135,21 @@ lt_status lt_batch_create(lt_context *ctx, const lt_request *reqs, int32_t nreqs
     *out = nullptr;
     std::lock_guard<std::mutex> lock(ctx->mu);
     cudaSetDevice(ctx->device);
-    /* the queue kernel variant nearest to the context's (tuned) FP32C Hessian shape */
-    const int variant = queue_variant(ctx->shape[LT_FP32C][OP_HESS]);
+    /* the tiles have the pixels per thread of the context's (tuned) FP32C Hessian shape */
+    const int shape = ctx->shape[LT_FP32C][OP_HESS];
+    long tiles = 0;
     std::vector<QSlot> host((size_t)nreqs);
     std::vector<double> cost((size_t)nreqs);
     for (int i = 0; i < nreqs; i++) {
         QSlot &s = host[i];
         memset(&s, 0, sizeof(s));
-        lt_status st = make_queue_item(ctx, &reqs[i], precision, nullptr, &s.item, shape_ppt(variant));
+        lt_status st = make_queue_item(ctx, &reqs[i], precision, nullptr, &s.item, shape_ppt(shape));
         if (st != LT_OK) {
             set_error(ctx, "request %d: %s", i, lt_last_error(ctx));
             return st;
         }
         cost[i] = (double)s.item.ntiles * (double)(reqs[i].cat->nhalos + 1);
+        tiles += s.item.ntiles;
     }
     /* costliest requests first: the queue runs them in order, so the cheap ones fill the
      * tail (longest-processing-time-first) */
@@ -162,7 +164,7 @@ lt_status lt_batch_create(lt_context *ctx, const lt_request *reqs, int32_t nreqs
     lt_batch *b = new (std::nothrow) lt_batch();
     if (!b) return LT_ERR_OUT_OF_MEMORY;
     b->mode = precision == LT_FP32C ? QMODE_C32 : QMODE_EXACT;
-    b->variant = variant;
+    b->variant = queue_variant(shape, tiles, ctx->num_sms);
     b->n = nreqs;
     b->bytes = sizeof(QSlot) * (size_t)nreqs + sizeof(QState);
     void *mem = nullptr;

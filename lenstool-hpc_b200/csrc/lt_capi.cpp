@@ -481,7 +481,7 @@ bool lt::grid_ok(const lt_grid *g)
 /* Run one grid evaluation: `kinds`/`outs` are the requested planes (host or device). */
 lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g, int precision, int op, int kmap,
                        double D, double mult, double scale, int nout, const int *kinds, double *const *outs,
-                       void *stream)
+                       void *stream, bool plain)
 {
     if (!ctx || !cat || !grid_ok(g) || nout < 1 || nout > LT_MAX_MAPS) {
         if (ctx) set_error(ctx, "invalid grid-call arguments");
@@ -537,6 +537,7 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
     a.mult = mult;
     a.scale = scale;
     a.status = ctx->status;
+    a.plain = plain;
     cudaStream_t s = (cudaStream_t)stream;
     const int side = call_side(ctx, cat, op, precision, a);
     /* the kernels of one band of rows (the whole grid for device outputs) */
@@ -621,7 +622,7 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
 
 int lt::call_side(const lt_context *ctx, const lt_catalog *cat, int op, int precision, const GridArgs &a)
 {
-    if (precision == LT_FP32C || cat->nhalos == 0) return 0;
+    if (precision == LT_FP32C || cat->nhalos == 0 || a.plain) return 0;
     if (precision == LT_FP64 && (op & OP_HESS)) op &= ~OP_HESS; /* every pair, in the reference's order */
     return op ? tree_side(cat, op, a.nx, a.ny, a.dx, a.dy, ctx->num_sms) : 0;
 }
@@ -825,7 +826,8 @@ lt_status lt_autotune(lt_context *ctx, const lt_catalog *cat, int32_t precision,
     }
     double *outs[2] = {planes, planes + (size_t)grid_n * grid_n};
     /* the search space: FP32C every built shape (pixels per thread, CTAs per SM, threads
-     * per CTA) with every stage size; the FP64 kernels their four (pixels, CTAs) shapes */
+     * per CTA) with every stage size; the FP64 kernels their four (pixels, CTAs) shapes;
+     * each itself, whatever replaces it on a small grid */
     std::vector<int> shapes;
     if (precision == LT_FP32C) {
         for (int k = 0; k < kNumShapes32; k++)
@@ -841,11 +843,11 @@ lt_status lt_autotune(lt_context *ctx, const lt_catalog *cat, int32_t precision,
     lt_status st = LT_OK;
     for (size_t k = 0; k < shapes.size() && st == LT_OK; k++) {
         ctx->shape[precision][sums] = shapes[k];
-        st = run_grid(ctx, cat, &g, precision, sums, 0, 1.0, 1.0, 1.0, nout, kinds, outs, nullptr);
+        st = run_grid(ctx, cat, &g, precision, sums, 0, 1.0, 1.0, 1.0, nout, kinds, outs, nullptr, true);
         if (st != LT_OK) break;
         cudaEventRecord(e0, nullptr);
         for (int rep = 0; rep < 2 && st == LT_OK; rep++)
-            st = run_grid(ctx, cat, &g, precision, sums, 0, 1.0, 1.0, 1.0, nout, kinds, outs, nullptr);
+            st = run_grid(ctx, cat, &g, precision, sums, 0, 1.0, 1.0, 1.0, nout, kinds, outs, nullptr, true);
         cudaEventRecord(e1, nullptr);
         if (st == LT_OK) st = lt_synchronize(ctx, nullptr);
         float ms = 0.f;

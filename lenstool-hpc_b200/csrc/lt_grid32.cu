@@ -386,12 +386,13 @@ static int launch_pass1(lt_context *ctx, const Fp32cCatalog &fc, int op, C32Args
      *   16.9      582 / 487 / 510                    1074 / 1027 / 1090
      *   27.7      818 / 763 / 788                    1518 / 1580 / 1709 */
     const double warps = ((A.g.nx + 15) / 16) * (double)((A.g.ny + 3) / 4) / (4. * ctx->num_sms);
-    if (P == 2 && warps <= (op == (OP_HESS | OP_POT) ? 1.6 : 10.)) {
+    const bool two = P == 2 && !A.g.plain;
+    if (two && warps <= (op == (OP_HESS | OP_POT) ? 1.6 : 10.)) {
         kern = small_kernel32(op);
         NT = kSmallThreads;
         cap = 64; /* 32 KB of stages */
         tiles(32, 4);
-    } else if (P == 2 && op == (OP_HESS | OP_POT) && warps <= 17.) {
+    } else if (two && op == (OP_HESS | OP_POT) && warps <= 17.) {
         kern = pick_kernel32(op, LT_SHAPE4(2, 3, 128, 64));
         NT = 128;
         cap = 64;

@@ -1,10 +1,12 @@
 /*
- * lt_grid64.cu -- FP64 persistent grid kernel: deflection, Hessian (+ map epilogue) and
- * potential sums over a packed halo catalogue.
+ * lt_grid64.cu -- FP64 persistent grid kernel over every halo x pixel pair: the Hessian in the
+ * reference's rounding sequence (+ map epilogue), the deflection, potential and fast Hessian of
+ * grids too small to gain from lt_tree64.cu, and the recomputation of a list of pixels.
  *
  * Work layout
- *   - A CTA of 256 threads owns a pixel tile of (32 P) x 8 pixels; each thread owns P
- *     adjacent pixels of one row (P = 2: one 16-byte store per output plane).
+ *   - A CTA of 256 threads owns a pixel tile of (32 P) x 8 pixels (64 threads, 16 x 4, for
+ *     small grids); each thread owns P adjacent pixels of one row (P = 2: one 16-byte store
+ *     per output plane).
  *   - CTAs are persistent: grid = resident CTAs per SM x SMs, tiles strided by gridDim.
  *   - The halo catalogue is walked in chunks of LT_CHUNK records (each chunk holds one
  *     profile type).  Chunk k+1 is brought into shared memory by one cp.async.bulk
@@ -222,7 +224,7 @@ static int launch_shape(int shape, const GridArgs &a, int num_sms, cudaStream_t 
 {
     /* a grid of less than two CTAs an SM: CTAs of 64 threads, one pixel each, so that it spreads
      * over all SMs, and (reference-order Hessian) two records a thread at a time */
-    if ((long)((a.nx + 31) / 32) * ((a.ny + 7) / 8) < 2 * num_sms)
+    if (!a.plain && (long)((a.nx + 31) / 32) * ((a.ny + 7) / 8) < 2 * num_sms)
         return launch_op<OP, 1, false, 4, kSmallThreads, 2>(a, num_sms, s);
     switch (shape) {
     case LT_SHAPE(1, 1): return launch_op<OP, 1, false, 1>(a, num_sms, s);
@@ -235,7 +237,7 @@ static int launch_shape(int shape, const GridArgs &a, int num_sms, cudaStream_t 
 int launch_grid64(int op, const GridArgs &args, int num_sms, void *stream, bool list_mode, int shape)
 {
     cudaStream_t s = (cudaStream_t)stream;
-    if (list_mode) { /* the FP32C recomputation pass: the out-of-line fast Hessian */
+    if (list_mode) { /* the FP32C recomputation pass */
         if (op != OP_HESS) return (int)cudaErrorInvalidValue;
         return launch_op<OP_HESS | OP_NI, 2, true, 2>(args, num_sms, s);
     }

@@ -113,7 +113,8 @@ bool is_device_pointer(const void *p);
 std::vector<lt_chunk> make_chunks(const int32_t *type, int n, int max_chunk, const double *dlsds = nullptr);
 
 lt_status run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g, int precision, int op, int kmap, double D,
-                   double mult, double scale, int nout, const int *kinds, double *const *outs, void *stream);
+                   double mult, double scale, int nout, const int *kinds, double *const *outs, void *stream,
+                   bool plain = false);
 /* far halos interpolated over tiles (lt_tree64.cu) */
 int tree_tables();
 int configure_tree64();

@@ -529,13 +529,13 @@ static QKern queue_kernel_for(int mode, int variant)
     }
 }
 
-/* The built variant nearest to an FP32C grid-kernel shape: its pixels per thread, and its
- * resident threads per SM rounded to 256 or 512. */
-int queue_variant(int shape32)
+/* The variant for an FP32C grid-kernel shape and `tiles` to run: the shape's pixels per thread,
+ * and registers for one CTA an SM where there are no more tiles than SMs, else for two.  B200,
+ * ms, two pixels a thread, two / one: 26 tiles of 200 halos 0.093 / 0.066, 512 tiles of 90 halos
+ * (mu) 0.200 / 0.213, 24 posterior models 11.1 / 14.4. */
+int queue_variant(int shape32, long tiles, int num_sms)
 {
-    const int ppt = shape_ppt(shape32) == 1 ? 1 : 2;
-    const int threads = shape_cps(shape32) * shape_threads(shape32);
-    return LT_SHAPE(ppt, threads > 384 ? 2 : 1);
+    return LT_SHAPE(shape_ppt(shape32) == 1 ? 1 : 2, tiles <= num_sms ? 1 : 2);
 }
 
 int queue_blocks(int mode, int variant, int num_sms)

@@ -67,7 +67,7 @@ struct QArgs {
 /* Persistent-kernel variants: the FP32C tiles come with 1 or 2 pixels per thread and
  * registers cut for 1 or 2 resident CTAs per SM (256 threads); `variant` is their
  * LT_SHAPE(pixels, CTAs).  The LT_FP64 tiles have one variant (2 CTAs per SM). */
-int queue_variant(int shape32);
+int queue_variant(int shape32, long tiles, int num_sms);
 int queue_blocks(int mode, int variant, int num_sms);
 int launch_queue(int mode, int variant, const QArgs &q, int blocks, cudaStream_t s);
 int launch_queue_reset(QSlot *slots, QState *state, int n, cudaStream_t s);

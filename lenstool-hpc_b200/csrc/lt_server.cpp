@@ -23,6 +23,7 @@
 #include <cmath>
 #include <atomic>
 #include <chrono>
+#include <climits>
 #include <condition_variable>
 #include <cstring>
 #include <deque>
@@ -570,7 +571,7 @@ lt_status lt_server_create(lt_context *ctx, const lt_server_config *cfg, lt_serv
     s->h_yield[0] = 1;
     s->h_yield[1] = 0;
     s->ring.assign((size_t)s->nslots, nullptr);
-    s->variant = queue_variant(ctx->shape[LT_FP32C][OP_HESS]);
+    s->variant = queue_variant(ctx->shape[LT_FP32C][OP_HESS], LONG_MAX, ctx->num_sms);
     s->blocks = queue_blocks(s->mode, s->variant, ctx->num_sms);
     {
         Extensions *x = ext_of(ctx);
