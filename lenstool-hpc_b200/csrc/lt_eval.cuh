@@ -334,16 +334,34 @@ __device__ __forceinline__ void eval64_chunk(const lt_rec64 *recs, const lt_nie6
     }
 }
 
-/* The FP32 terms of one record at a thread's pixels (halo-frame offsets u, v) added to the
- * block sums. */
+/* The FP32 terms of one record at a thread's pixels (halo-frame offsets u, v), and their addition
+ * to the block sums. */
+template <int P>
+struct Terms1 {
+    KG32 h[P];
+    G32 g[P];
+    float p[P];
+};
 template <int OP, int P, int TYPE>
-__device__ __forceinline__ void terms32(const lt_rec32 &r, const float (&u)[P], const float (&v)[P], Acc32<P> &acc)
+__device__ __forceinline__ Terms1<P> terms32(const lt_rec32 &r, const float (&u)[P], const float (&v)[P])
 {
+    Terms1<P> t;
 #pragma unroll
     for (int k = 0; k < P; k++) {
         const Nie32 n = nie32<TYPE>(r, u[k], v[k]);
+        if (OP & OP_HESS) t.h[k] = hess32<TYPE>(r, u[k], v[k], n);
+        if (OP & (OP_GRAD | OP_POT)) t.g[k] = grad32<TYPE>(r, u[k], v[k], n);
+        if (OP & OP_POT) t.p[k] = pot32<TYPE>(r, u[k], v[k], n, t.g[k]);
+    }
+    return t;
+}
+template <int OP, int P>
+__device__ __forceinline__ void add32(const lt_rec32 &r, const Terms1<P> &s, Acc32<P> &acc)
+{
+#pragma unroll
+    for (int k = 0; k < P; k++) {
         if (OP & OP_HESS) {
-            const KG32 t = hess32<TYPE>(r, u[k], v[k], n);
+            const KG32 &t = s.h[k];
             acc.bk.set(k, __fadd_rn(acc.bk.get(k), t.k));
             acc.bg1.set(k, __fmaf_rn(t.g1, r.c2t, __fmaf_rn(-t.g2, r.s2t, acc.bg1.get(k))));
             acc.bg2.set(k, __fmaf_rn(t.g1, r.s2t, __fmaf_rn(t.g2, r.c2t, acc.bg2.get(k))));
@@ -351,19 +369,15 @@ __device__ __forceinline__ void terms32(const lt_rec32 &r, const float (&u)[P], 
             acc.mk.set(k, __fmaf_rn(t.k, t.k, acc.mk.get(k)));
             acc.mg.set(k, __fmaf_rn(ag, ag, acc.mg.get(k)));
         }
-        if (OP & (OP_GRAD | OP_POT)) {
-            const G32 t = grad32<TYPE>(r, u[k], v[k], n);
-            if (OP & OP_GRAD) {
-                acc.bgx.set(k, __fmaf_rn(t.x, r.cs, __fmaf_rn(-t.y, r.sn, acc.bgx.get(k))));
-                acc.bgy.set(k, __fmaf_rn(t.y, r.cs, __fmaf_rn(t.x, r.sn, acc.bgy.get(k))));
-            }
-            if (OP & OP_POT) acc.bp.set(k, __fadd_rn(acc.bp.get(k), pot32<TYPE>(r, u[k], v[k], n, t)));
+        if (OP & OP_GRAD) {
+            acc.bgx.set(k, __fmaf_rn(s.g[k].x, r.cs, __fmaf_rn(-s.g[k].y, r.sn, acc.bgx.get(k))));
+            acc.bgy.set(k, __fmaf_rn(s.g[k].y, r.cs, __fmaf_rn(s.g[k].x, r.sn, acc.bgy.get(k))));
         }
+        if (OP & OP_POT) acc.bp.set(k, __fadd_rn(acc.bp.get(k), s.p[k]));
     }
 }
 
-/* terms32 of a cut dPIE at two pixels, packed: the same operations and roundings, the terms and
- * their addition to the block sums apart. */
+/* The same of a cut dPIE at two pixels, packed: the same operations and roundings. */
 struct Terms2 {
     KG2 h;
     G2 g;
@@ -412,6 +426,18 @@ __device__ __forceinline__ void frame32x2(const lt_rec32 &r, const double (&px)[
     v = fma(dup(ty), dup(r.cs), mul(t, dup(-r.sn)));
 }
 
+template <int P>
+__device__ __forceinline__ void frame32(const lt_rec32 &r, const double (&px)[P], double py, float (&u)[P], float (&v)[P])
+{
+    const float ty = __double2float_rn(__dsub_rn(py, r.y0));
+#pragma unroll
+    for (int k = 0; k < P; k++) {
+        const float tx = __double2float_rn(__dsub_rn(px[k], r.x0));
+        u[k] = __fmaf_rn(tx, r.cs, __fmul_rn(ty, r.sn));
+        v[k] = __fmaf_rn(ty, r.cs, -__fmul_rn(tx, r.sn));
+    }
+}
+
 /* One FP32 record at the pixels px[0..P) of row py, in FP64 if its disc reaches the warp. */
 template <int OP, int P, int TYPE>
 __device__ __forceinline__ void eval32_record(const lt_rec32 &r, bool maybe_near, const lt_rec64 *recs64,
@@ -425,13 +451,7 @@ __device__ __forceinline__ void eval32_record(const lt_rec32 &r, bool maybe_near
         frame32x2(r, px, py, u2, v2);
         u[0] = p2::lo(u2), u[1] = p2::hi(u2), v[0] = p2::lo(v2), v[1] = p2::hi(v2);
     } else {
-        const float ty = __double2float_rn(__dsub_rn(py, r.y0));
-#pragma unroll
-        for (int k = 0; k < P; k++) {
-            const float tx = __double2float_rn(__dsub_rn(px[k], r.x0));
-            u[k] = __fmaf_rn(tx, r.cs, __fmul_rn(ty, r.sn));
-            v[k] = __fmaf_rn(ty, r.cs, -__fmul_rn(tx, r.sn));
-        }
+        frame32<P>(r, px, py, u, v);
     }
     bool near = false;
     if (maybe_near) {
@@ -457,13 +477,13 @@ __device__ __forceinline__ void eval32_record(const lt_rec32 &r, bool maybe_near
     } else if constexpr (packed) {
         add32x2<OP>(r, terms32x2<OP, true>(r, u2, v2), acc);
     } else {
-        terms32<OP, P, TYPE>(r, u, v, acc);
+        add32<OP, P>(r, terms32<OP, P, TYPE>(r, u, v), acc);
     }
 }
 
 /* One chunk of FP32 records (at most 128) for the pixels px[0..P) of row py, the lane's
  * pixels (ix .. ix + P - 1, iy) of grid `a`.  Every record of an FP32C chunk has the same
- * Kmap weight.  With U = 2 the terms of two cut dPIE records interleave and are added in their
+ * Kmap weight.  With U = 2 the terms of two records interleave and are added in their
  * order (small grids, where one record's chain at a time leaves the SM idle). */
 template <int OP, int P, int TYPE, int U = 1>
 __device__ __forceinline__ void eval32_chunk(const lt_rec32 *recs, const lt_rec64 *recs64, const lt_nie64 *nie, int count,
@@ -490,6 +510,20 @@ __device__ __forceinline__ void eval32_chunk(const lt_rec32 *recs, const lt_rec6
                     if ((h & (kBlock32 - 1)) == kBlock32 - 1) fold32<OP, P>(acc, wchunk);
                     h++;
                     add32x2<OP>(recs[h], t1, acc);
+                    if ((h & (kBlock32 - 1)) == kBlock32 - 1) fold32<OP, P>(acc, wchunk);
+                    continue;
+                }
+            } else if constexpr (U == 2 && P == 2) {
+                if (h + 1 < h0 + n && ((mask >> (h - h0)) & 3ull) == 0) {
+                    float u[2][P], v[2][P];
+                    frame32<P>(recs[h], px, py, u[0], v[0]);
+                    frame32<P>(recs[h + 1], px, py, u[1], v[1]);
+                    const Terms1<P> t0 = terms32<OP, P, TYPE>(recs[h], u[0], v[0]);
+                    const Terms1<P> t1 = terms32<OP, P, TYPE>(recs[h + 1], u[1], v[1]);
+                    add32<OP, P>(recs[h], t0, acc);
+                    if ((h & (kBlock32 - 1)) == kBlock32 - 1) fold32<OP, P>(acc, wchunk);
+                    h++;
+                    add32<OP, P>(recs[h], t1, acc);
                     if ((h & (kBlock32 - 1)) == kBlock32 - 1) fold32<OP, P>(acc, wchunk);
                     continue;
                 }

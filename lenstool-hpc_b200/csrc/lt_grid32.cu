@@ -377,23 +377,29 @@ static int launch_pass1(lt_context *ctx, const Fp32cCatalog &fc, int op, C32Args
         A.g.ntiles = A.g.tiles_x * ((A.g.ny + h - 1) / h);
     };
     tiles(32 * P, NT / 32);
-    /* Grids of few warps per scheduler (two-pixel shapes), 300 halos, us:
-     *   warps     Hessian 256 / 128 x 2 / 64 x 2     lens maps 256 / 128 x 2 (3 CTAs) / 64 x 2
-     *    1.3      85 / 74 / 72                       160 / 138 / 138
-     *    2.7      126 / 96 / 95                      236 / 187 / 217
-     *    5.5      241 / 195 / 178                    446 / 396 / 381
-     *    9.6      355 / 291 / 283                    658 / 608 / 622
-     *   16.9      582 / 487 / 510                    1074 / 1027 / 1090
-     *   27.7      818 / 763 / 788                    1518 / 1580 / 1709 */
+    /* Grids of few warps per scheduler take CTAs of 64 threads; the lens maps, whose 256-thread CTAs
+     * (one record at a time) run in waves of 4 warps a scheduler, take 128 threads and two records
+     * at a time where the last wave would be less than 60% full.  B200, 300 halos, us:
+     *   warps   Hessian 256 / 128 x 2 / 64 x 2     lens maps 256 / 128 x 2 / 64 x 2
+     *    0.8      88 / 74 / 60                       165 / 146 / 104
+     *    2.8     128 / 117 / 95                      233 / 239 / 215
+     *    4.8     188 / 168 / 178                     351 / 344 / 378
+     *    7.2     242 / 226 / 229                     450 / 471 / 501
+     *   10.8     358 / 330 / 346                     669 / 689 / 731
+     *   16.9     587 / 488 / 512                    1097 / 1027 / 1105
+     *   26.2     821 / 768 / 770                    1537 / 1614 / 1630
+     *   32.0    1048 / 918 / 935                    1959 / 1932 / 1994
+     * deflection and potential like the Hessian; profiles of types 5 and 8 among the halos shift
+     * all columns alike but the last, which loses up to 12% (lens maps 36%) above 4 warps. */
     const double warps = ((A.g.nx + 15) / 16) * (double)((A.g.ny + 3) / 4) / (4. * ctx->num_sms);
-    const bool two = P == 2 && !A.g.plain;
-    if (two && warps <= (op == (OP_HESS | OP_POT) ? 1.6 : 10.)) {
+    const bool two = P == 2 && !A.g.plain, lens = op == (OP_HESS | OP_POT);
+    if (two && warps <= (lens ? 1.6 : 4.)) {
         kern = small_kernel32(op);
         NT = kSmallThreads;
         cap = 64; /* 32 KB of stages */
         tiles(32, 4);
-    } else if (two && op == (OP_HESS | OP_POT) && warps <= 17.) {
-        kern = pick_kernel32(op, LT_SHAPE4(2, 3, 128, 64));
+    } else if (two && lens && warps < 3.6 * std::ceil(warps / 4.)) {
+        kern = pick_kernel32(op, LT_SHAPE4(2, 4, 128, 64));
         NT = 128;
         cap = 64;
         tiles(64, 4);

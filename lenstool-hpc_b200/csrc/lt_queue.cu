@@ -213,10 +213,10 @@ __device__ __noinline__ bool tile32(const QItem &it, int tile, Stage &st, int32_
                                       eval32_chunk<OP, P, 81, OP == (OP_HESS | OP_POT) ? 1 : 2>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
                                       break;
                                   case 8:
-                                      eval32_chunk<OP, P, 8>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
+                                      eval32_chunk<OP, P, 8, OP == (OP_HESS | OP_POT) ? 1 : 2>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
                                       break;
                                   case 5:
-                                      eval32_chunk<OP, P, 5>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
+                                      eval32_chunk<OP, P, 5, OP == (OP_HESS | OP_POT) ? 1 : 2>(recs, a.recs, a.nie, c.count, px, py, a, ix, iy, acc);
                                       break;
                                   default: break;
                                   }

@@ -1,6 +1,7 @@
-"""The FP32C pair loop of two pixels a thread evaluates a cut dPIE in packed form; with one pixel a
-thread it takes the scalar form.  Both round every operation alike, so the planes of the two shapes are equal wherever no FP64 disc is near (a warp of each
-shape covers another box, and a disc sends the whole box to FP64)."""
+"""The FP32C pair loop of two pixels a thread evaluates a cut dPIE in packed form, and in small CTAs two
+records of any type at a time; with one pixel a thread it takes the scalar form, record by record.  All
+round every operation alike, so the planes of the shapes are equal wherever no FP64 disc is near (a warp
+of each shape covers another box, and a disc sends the whole box to FP64)."""
 import numpy as np
 import pytest
 
@@ -34,10 +35,11 @@ def _maps(ctx, cat, g, config):
 
 @pytest.mark.parametrize("n", [1, 7, 8, 9, 63, 65, 130, 257])
 @pytest.mark.parametrize("grid", [(96, 64), (65, 41), (1, 7), (130, 1)])
-def test_packed_equals_scalar(ctx, n, grid):
+@pytest.mark.parametrize("types", [[81], [8], [5], [5, 8, 81]])
+def test_packed_equals_scalar(ctx, n, grid, types):
     rng = np.random.default_rng(n)
     # every halo and its disc left of the field
-    cat = catalog.make_catalog([81] * n, rng.uniform(-200., -120., n), rng.uniform(-90., 90., n),
+    cat = catalog.make_catalog(sorted((types * n)[:n]), rng.uniform(-200., -120., n), rng.uniform(-90., 90., n),
                                rng.uniform(80., 200., n), rng.uniform(0.05, 0.5, n), rng.uniform(0., np.pi, n),
                                rng.uniform(0.05, 0.2, n), rng.uniform(1., 300., n))
     nx, ny = grid

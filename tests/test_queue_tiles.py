@@ -27,7 +27,9 @@ def ctx():
 @pytest.mark.parametrize("order", ["large first", "repeated"])
 def test_batch_equals_single_calls(ctx, halos, order):
     import torch
-    cat = ctx.upload(catalog.cluster_galaxy_catalog(2, halos - 2, 5))
+    cat = catalog.cluster_galaxy_catalog(2, halos - 2, 5)
+    cat.type = np.sort(np.random.default_rng(halos).choice(np.array([5, 8, 81, 81], np.int32), halos))
+    cat = ctx.upload(cat)
     sides = SIDES if order == "large first" else [SIDES[3]] * 9 + [SIDES[0]] * 40
     grids = [catalog.Grid(-60., 60., -60. * ny / nx, 60. * ny / nx, nx, ny) for nx, ny in sides]
     new = lambda g: {k: torch.full((g.ny, g.nx), np.nan, dtype=torch.float64, device="cuda") for k in ("kappa", "mu")}
