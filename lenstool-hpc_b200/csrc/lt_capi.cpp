@@ -565,7 +565,7 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
      * whole grid and the maps are the same bit for bit. */
     int band = (int)(((long)g->ny + kHostBands - 1) / kHostBands);
     if (band < kMinBandRows) band = kMinBandRows;
-    const int tile_rows = side ? 2 * side : 8;
+    const int tile_rows = side ? tree_rows(side) : 8;
     band = (band + tile_rows - 1) / tile_rows * tile_rows;
     if (!ctx->copy_stream) {
         cudaError_t e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);

@@ -117,6 +117,7 @@ lt_status run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g, int
                    bool plain = false);
 /* far halos interpolated over tiles (lt_tree64.cu) */
 int tree_tables();
+int tree_rows(int side);
 int configure_tree64();
 int tree_side(const lt_catalog *cat, int op, int nx, int ny, double dx, double dy, int num_sms);
 int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side, void *stream);

@@ -23,8 +23,9 @@
  * shear 3e-15 at 4.0.  A far term is ~1% of its sum, so the truncation stays below the sum's own
  * rounding.
  *
- * Layout.  One CTA of 256 threads a tile, a cluster of four CTAs a parent.  A CTA sorts the
- * halos into lists, a halo a thread: its quarter of those far from the parent, those far from its
+ * Layout.  One CTA of 256 threads a tile, a cluster of four CTAs a parent (two and eight for a
+ * grid of few tiles: half of the tile's far halos and of its passes each).  A CTA sorts the
+ * halos into lists, a halo a thread: its share of those far from the parent, those far from its
  * tile only, those near it; the listed records are gathered in shared memory, 128 at a time, and
  * each thread sums them at one node of the parent, then of the tile, two records at a time.  The
  * four shares of the parent's node values are read from the cluster's shared memory and
@@ -51,6 +52,7 @@ constexpr int kNodes = 16;
 constexpr int kStage = 128;  /* records staged at once */
 constexpr int kRound = 1024; /* halos classified between two walks */
 constexpr int kNearBlock = 8;
+constexpr int kSplit = 1024;    /* tree_side()'s mark of two CTAs a tile */
 constexpr int kNearList = 2048; /* near halos of a tile; a tile with more evaluates every halo */
 
 /* Tile sides, and per side T the Lagrange basis of the nodes: L[i][c] at pixel c of the tile, and
@@ -185,10 +187,10 @@ __device__ __forceinline__ void tree_two(int type, const lt_nie64 &r0, const lt_
 }
 
 /* The pixels of a tile: the interpolated far sums and its near halos, two pixels a thread a pass. */
-template <int OP>
+template <int OP, int N>
 __device__ __forceinline__ void tree_pixels(const TreeArgs &A, unsigned char *smem, int32_t *s_type,
-                                            const int32_t *list, int near, int tx0, int ty0, const double *F, double *H,
-                                            const double *L)
+                                            const int32_t *list, int near, int tx0, int ty0, int part, const double *F,
+                                            double *H, const double *L)
 {
     constexpr int NQ = TreeOp<OP>::planes;
     const GridArgs &a = A.g;
@@ -206,7 +208,7 @@ __device__ __forceinline__ void tree_pixels(const TreeArgs &A, unsigned char *sm
     };
     if (near <= kStage) gather(0, near);
 
-    for (int r0 = 0; r0 < T && ty0 + r0 < a.ny; r0 += rows) {
+    for (int r0 = part * rows; r0 < T && ty0 + r0 < a.ny; r0 += N * rows) {
         __syncthreads(); /* F and the gathered records; H is free */
         for (int e = tid; e < NQ * rows * kNodes; e += kTreeThreads) {
             const int q = e / (rows * kNodes), r = (e / kNodes) % rows, i = e % kNodes;
@@ -327,8 +329,9 @@ struct Square {
     }
 };
 
-template <int OP>
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kTreeThreads, 2) tree64_kernel(const TreeArgs A)
+/* N CTAs a tile, 4 N a cluster. */
+template <int OP, int N>
+__global__ void __launch_bounds__(kTreeThreads, 2) tree64_kernel(const TreeArgs A)
 {
     constexpr int NQ = TreeOp<OP>::planes, NN = kNodes * kNodes;
     const GridArgs &a = A.g;
@@ -344,15 +347,17 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kTreeThreads, 2) tre
     int32_t *list = reinterpret_cast<int32_t *>(L + kNodes * T);              /* near halos */
     int32_t *own = list + kNearList, *share = own + kRound;                   /* far halos of a round */
 
-    const int tid = threadIdx.x, rank = blockIdx.x & 3;
+    constexpr int size = 4 * N;
+    const int tid = threadIdx.x;
+    const int rank = blockIdx.x & (size - 1), tile = rank & 3, part = rank >> 2;
     for (int e = tid; e < kNodes * T; e += kTreeThreads) L[e] = g_lagrange[A.table + e];
     const double node_x = g_nodes[tid & 15], node_y = g_nodes[tid >> 4];
 
     /* rows of clusters from the middle outwards: the halos crowd there, and the dear tiles go first */
-    const int ccols = (a.tiles_x + 1) / 2, crows = (int)gridDim.x / (4 * ccols), cl = (int)blockIdx.x >> 2;
+    const int ccols = (a.tiles_x + 1) / 2, crows = (int)gridDim.x / (size * ccols), cl = (int)blockIdx.x / size;
     const int r = cl / ccols, crow = (crows - 1) / 2 + ((r & 1) ? (r + 1) / 2 : -(r / 2));
     const int px0 = 2 * T * (cl % ccols), py0 = 2 * T * crow;
-    const int tx0 = px0 + (rank & 1) * T, ty0 = py0 + (rank >> 1) * T;
+    const int tx0 = px0 + (tile & 1) * T, ty0 = py0 + (tile >> 1) * T;
     const bool alive = tx0 < a.nx && ty0 < a.ny; /* a tile beyond the grid does its share only */
     const Square P(a, px0, py0, 2 * T, TreeOp<OP>::far), C(a, tx0, ty0, T, TreeOp<OP>::far);
 
@@ -361,7 +366,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kTreeThreads, 2) tre
     int near = 0;
     for (int base = 0; base < A.nhalos; base += kRound) {
         /* the round's halos to the lists, in the catalogue's order: far from the parent (this
-         * CTA's quarter of them), far from the tile only, near */
+         * CTA's share of them), far from the tile only (all, or this CTA's half), near */
         int nshare = 0, nown = 0;
         for (int sub = 0; sub < kRound && base + sub < A.nhalos; sub += kTreeThreads) {
             const int i = base + sub + tid;
@@ -371,9 +376,9 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kTreeThreads, 2) tre
                 const bool point = A.types[i] == 5;
                 const double x = h.x0, y = h.y0, q2 = point ? h.q2 / h.k : h.q2, s = point ? 0. : h.sc;
                 if (P.is_far(x, y, q2, s * s))
-                    cls = (i & 3) == rank ? 0 : -1;
+                    cls = (i & (size - 1)) == rank ? 0 : -1;
                 else if (alive)
-                    cls = C.is_far(x, y, q2, s * s) ? 1 : 2;
+                    cls = !C.is_far(x, y, q2, s * s) ? 2 : (i & (N - 1)) == part ? 1 : -1;
             }
             int at[3], tot[3];
             int (*cnt)[kTreeThreads / 32] = s_cnt[(sub / kTreeThreads) & 1];
@@ -428,17 +433,23 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kTreeThreads, 2) tre
     cluster_arrive();
     cluster_wait();
     double *PP = reinterpret_cast<double *>(stage), *G = PP + NQ * NN; /* [plane][j][i] */
+    double far_sum[NQ]; /* the tile's far halos at this node */
 #pragma unroll
     for (int q = 0; q < NQ; q++) {
-        double v[4];
+        double v[size];
 #pragma unroll
-        for (int k = 0; k < 4; k++) v[k] = cluster_load(S + q * NN + tid, k);
+        for (int k = 0; k < size; k++) v[k] = cluster_load(S + q * NN + tid, k);
+        if (N == 2) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[k] += v[(k + 4) % size];
+            far_sum[q] = cluster_load(F + q * NN + tid, tile) + cluster_load(F + q * NN + tid, tile + 4);
+        }
         PP[q * NN + tid] = (v[0] + v[1]) + (v[2] + v[3]);
     }
-    cluster_arrive(); /* the shares are read: waited for before the exit */
+    cluster_arrive(); /* the shares are read: waited for before the exit and, N = 2, before F changes */
     if (alive) {
         __syncthreads();
-        const double *bx = g_parent + A.parent + (rank & 1) * NN, *by = g_parent + A.parent + (rank >> 1) * NN;
+        const double *bx = g_parent + A.parent + (tile & 1) * NN;
 #pragma unroll
         for (int q = 0; q < NQ; q++) {
             double g = 0.;
@@ -447,29 +458,43 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kTreeThreads, 2) tre
                 g = fma(bx[i * kNodes + (tid & 15)], PP[q * NN + (tid & ~15) + i], g);
             G[q * NN + tid] = g;
         }
+    }
+    if (N == 2) cluster_wait();
+    if (alive) {
         __syncthreads();
+        const double *by = g_parent + A.parent + (tile >> 1) * NN;
 #pragma unroll
         for (int q = 0; q < NQ; q++) {
             double g = 0.;
 #pragma unroll
             for (int j = 0; j < kNodes; j++)
                 g = fma(by[j * kNodes + (tid >> 4)], G[q * NN + j * kNodes + (tid & 15)], g);
-            F[q * NN + tid] += g;
+            F[q * NN + tid] = (N == 2 ? far_sum[q] : F[q * NN + tid]) + g;
         }
         __syncthreads(); /* F; the stage is free */
-        tree_pixels<OP>(A, smem, s_type, list, near, tx0, ty0, F, H, L);
+        tree_pixels<OP, N>(A, smem, s_type, list, near, tx0, ty0, part, F, H, L);
     }
-    cluster_wait();
+    if (N == 1) cluster_wait();
 }
 
-template <int OP>
+template <int OP, int N>
 static int launch_tree_op(TreeArgs &A, cudaStream_t s)
 {
-    const size_t smem = tree_smem<OP>(A.T);
     const int clusters = ((A.g.tiles_x + 1) / 2) * ((A.g.ntiles / A.g.tiles_x + 1) / 2);
-    tree64_kernel<OP><<<4 * clusters, kTreeThreads, smem, s>>>(A);
+    cudaLaunchAttribute cluster = {};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = 4 * N;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(4 * N * clusters);
+    c.blockDim = dim3(kTreeThreads);
+    c.dynamicSmemBytes = tree_smem<OP>(A.T);
+    c.stream = s;
+    c.attrs = &cluster;
+    c.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&c, tree64_kernel<OP, N>, (const TreeArgs)A);
     count_launch(1);
-    return (int)cudaGetLastError();
+    return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
 int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side, void *stream)
@@ -478,7 +503,9 @@ int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side,
     A.g = args;
     A.types = reinterpret_cast<const Fp32cCatalog *>(&cat->aux_desc)->types;
     A.nhalos = cat->nhalos;
-    A.T = side;
+    A.T = side & (kSplit - 1);
+    const bool two = side & kSplit;
+    side = A.T;
     A.table = A.parent = 0;
     for (int T : kSides) {
         if (T == side) break;
@@ -489,13 +516,16 @@ int launch_tree64(const lt_catalog *cat, int op, const GridArgs &args, int side,
     A.g.ntiles = A.g.tiles_x * ((args.ny + side - 1) / side);
     cudaStream_t s = (cudaStream_t)stream;
     switch (op) {
-    case OP_GRAD: return launch_tree_op<OP_GRAD>(A, s);
-    case OP_POT: return launch_tree_op<OP_POT>(A, s);
-    case OP_HESS: return launch_tree_op<OP_HESS>(A, s);
-    case OP_HESS | OP_POT: return launch_tree_op<OP_HESS | OP_POT>(A, s);
+    case OP_GRAD: return two ? launch_tree_op<OP_GRAD, 2>(A, s) : launch_tree_op<OP_GRAD, 1>(A, s);
+    case OP_POT: return two ? launch_tree_op<OP_POT, 2>(A, s) : launch_tree_op<OP_POT, 1>(A, s);
+    case OP_HESS: return two ? launch_tree_op<OP_HESS, 2>(A, s) : launch_tree_op<OP_HESS, 1>(A, s);
+    case OP_HESS | OP_POT: return two ? launch_tree_op<OP_HESS | OP_POT, 2>(A, s) : launch_tree_op<OP_HESS | OP_POT, 1>(A, s);
     default: return (int)cudaErrorInvalidValue;
     }
 }
+
+/* Rows of a cluster of tiles. */
+int tree_rows(int side) { return 2 * (side & (kSplit - 1)); }
 
 /* The tile side for sums `op` of a grid, or 0 where the direct kernels are the faster: costs in
  * pairs per resident CTA (two an SM), fitted to 54 measured combinations of sum, grid (96^2 to
@@ -534,7 +564,13 @@ int tree_side(const lt_catalog *cat, int op, int nx, int ny, double dx, double d
             side = T;
         }
     }
-    return side;
+    /* Two CTAs a tile where the tiles are fewer than the resident CTAs and dear enough for the
+     * second's lists and interpolation.  B200, us, one / two: potential of 200 halos on 512^2 (256
+     * tiles of 32) 179 / 162, of 400 on 400^2 340 / 313; deflection of 1000 on 500^2 538 / 501, on
+     * 256^2 (256 tiles of 16, whose one pass is not shared) 538 / 455, but of 200 on 256^2 74 / 94,
+     * of 10 on 400^2 21 / 32, of 300 on 800^2 (676 tiles) 246 / 273. */
+    const double tiles = side ? 4. * std::ceil(nx / (2. * side)) * std::ceil(ny / (2. * side)) : 0.;
+    return side && tiles <= slots && n >= (side > 16 ? 40 : 500) ? side | kSplit : side;
 }
 
 template <int OP>
@@ -542,7 +578,9 @@ static cudaError_t allow_smem()
 {
     size_t most = 0;
     for (int T : kSides) most = std::max(most, tree_smem<OP>(T));
-    return cudaFuncSetAttribute(tree64_kernel<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    const cudaError_t e = cudaFuncSetAttribute(tree64_kernel<OP, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(tree64_kernel<OP, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
 /* Once per context: the kernels' shared memory on the current device. */
