@@ -17,7 +17,7 @@
  * rho^-16 with rho the sum of the semi-axes of the largest regular ellipse around the tile, so a
  * halo is far when
  *   q^2 (max(0, d - diagonal/2)^2 + s^2) >= (kFar h)^2,
- * d from the tile's centre, h the larger half width.  kFar is taken per sum from the measured
+ * d from the tile's centre, h the larger half width, and lies outside the circle around the tile.  kFar is taken per sum from the measured
  * error of one term against extended precision (q 0.4 to 0.9, random orientation, core and cut
  * radii; relative to the term): deflection 5e-15 at 3.2, potential 2e-16 at 3.0, convergence and
  * shear 3e-15 at 4.0.  A far term is ~1% of its sum, so the truncation stays below the sum's own
@@ -318,14 +318,15 @@ struct Square {
         yc = 0.5 * (y0 + y1);
         hx = 0.5 * (x1 - x0);
         hy = 0.5 * (y1 - y0);
-        diag = sqrt(hx * hx + hy * hy);
+        diag = 1.0001 * sqrt(hx * hx + hy * hy); /* the corners' pixels inside */
         const double r = far * fmax(fabs(hx), fabs(hy));
         reach2 = r * r;
     }
     __device__ __forceinline__ bool is_far(double x, double y, double q2, double s2) const
     {
         const double dx = x - xc, dy = y - yc, d = fmax(sqrt(dx * dx + dy * dy) - diag, 0.);
-        return q2 * (d * d + s2) >= reach2;
+        /* d = 0: a halo inside is near whatever its core, for at its centre the potential is 0/0 */
+        return d > 0. && q2 * (d * d + s2) >= reach2;
     }
 };
 

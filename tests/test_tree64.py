@@ -108,6 +108,28 @@ def test_fast_lens_maps_against_extended_precision(ctx, e, kmap):
         assert max_rel_err(ctx.lens_maps(cat, g, precision="fp64", which=("psi",))["psi"].ravel()[idx], ref[3]) <= TOL
 
 
+@pytest.mark.parametrize("rcore", [0.1, 15., 60.])
+def test_halo_centre_on_a_pixel(ctx, rcore):
+    """The potential is 0/0 at a centre, in a core wider than the tile too: NaN where the batch has it."""
+    n = 200
+    rng = np.random.default_rng(5)
+    cat = catalog.make_catalog([81] * n, np.r_[0., 25., rng.uniform(-90., 90., n - 2)],
+                               np.r_[0., -50., rng.uniform(-90., 90., n - 2)], rng.uniform(80., 300., n),
+                               rng.uniform(0.05, 0.5, n), rng.uniform(0., np.pi, n), np.r_[rcore, rcore, np.full(n - 2, 0.1)],
+                               np.full(n, 200.))
+    g = catalog.Grid(-100., 100., -100., 100., 641, 641)  # steps of 0.3125
+    want = _direct(ctx, cat, g, ["deflection_x", "deflection_y", "potential"], 1.0)
+    ax, ay, psi = _dev(g), _dev(g), _dev(g)
+    ctx.gradient_grid(cat, g, out=(ax, ay))
+    ctx.potential_grid(cat, g, out=psi)
+    ctx.synchronize()
+    for got, k in ((ax, "deflection_x"), (ay, "deflection_y"), (psi, "potential")):
+        got, ok = got.cpu().numpy(), np.isfinite(want[k])
+        assert np.array_equal(np.isfinite(got), ok), k
+        assert max_rel_err(np.where(ok, got, 0.), np.where(ok, want[k], 0.)) <= TOL, k
+    assert np.isnan(want["potential"][320, 320])
+
+
 @pytest.mark.parametrize("n", [129, 2049, 4000])
 def test_many_near_halos(ctx, n):
     """Halos crowded into one tile: more of them near than are staged at once (128), and more
