@@ -198,7 +198,7 @@ __device__ __forceinline__ void defl64(const lt_nie64 &h, const Nie64 &n, double
         qv = TYPE == 8 ? lo : mul(lo, add(add(n.pt, h.q2st), kv));
     }
     au = mul(h.Ak, atan_quot(nu, du));
-    av = copysign(mul(h.hAk, log1p_quot(add(nv, nv), qv)), n.v);
+    av = mul(h.hAk, copysign(log1p_quot(add(nv, nv), qv), n.v)); /* hAk < 0: a halo of negative mass */
 }
 
 /* Adds one pair's deflection in the sky frame. */
