@@ -78,6 +78,11 @@ __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, 
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+/* a, negated where b is negative */
+__device__ __forceinline__ double flip(double a, double b)
+{
+    return __hiloint2double(__double2hiint(a) ^ (__double2hiint(b) & (int)0x80000000), __double2loint(a));
+}
 /* a positive normal float (or +0, as 2^-127) as a double, by its bits */
 __device__ __forceinline__ double widen(int bits) { return __hiloint2double((bits >> 3) + 0x38000000, 0); }
 } // namespace c64
@@ -86,8 +91,9 @@ __device__ __forceinline__ double widen(int bits) { return __hiloint2double((bit
  * next to a (chosen in FP32: any neighbouring point would do),
  *   atan a = atan c + atan t,  t = (min - c max)/(max + c min),  |t| <= 1/128,
  * and atan t = t - t^3/3 + t^5/5 - t^7/7 (truncation t^9/9 < 2e-18 of t).  One reciprocal,
- * 12 FP64 operations; within 2 ulp of atan(n/d).  j = 0 leaves t = a exactly, so small
- * quotients keep their relative accuracy. */
+ * 12 FP64 operations; within 2 ulp of atan(n/d) while the larger of |n| and d is within FP32's
+ * range (lengths of 1e-19 to 1e19 arcsec; longer cut radii do not enter, pack_nie64).  j = 0
+ * leaves t = a exactly, so small quotients keep their relative accuracy. */
 __device__ __forceinline__ double atan_quot(double n, double d)
 {
     using namespace c64;
@@ -95,7 +101,7 @@ __device__ __forceinline__ double atan_quot(double n, double d)
     const float nf = __double2float_rn(an), df = __double2float_rn(d);
     const bool swap = nf > df;
     const double mn = swap ? d : an, mx = swap ? an : d;
-    const float af = fminf(__fmul_rn(fminf(nf, df), frcp(fmaxf(nf, df))), 1.f);
+    const float af = __saturatef(__fmul_rn(fminf(nf, df), frcp(fmaxf(nf, df)))); /* 0/0 (below 2^-126): 0 */
     const float jf = __fmaf_rn(af, 64.f, 12582912.f); /* 1.5 x 2^23 + j */
     const int j = __float_as_int(jf) & 127;
     const double c = j ? widen(__float_as_int(__fmul_rn(__fsub_rn(jf, 12582912.f), 0.015625f))) : 0.;
@@ -115,7 +121,7 @@ __device__ __forceinline__ double atan_quot(double n, double d)
 __device__ __forceinline__ double log1p_quot(double n, double d)
 {
     using namespace c64;
-    const float m = fminf(__fmaf_rn(__double2float_rn(n), frcp(__double2float_rn(d)), 1.f), 0x1p126f);
+    const float m = fmaxf(__fmaf_rn(__double2float_rn(n), frcp(__double2float_rn(d)), 1.f), 1.f); /* 0/0: 1 */
     const int b = (__float_as_int(m) + 0x10000) & 0x7ffe0000;
     const double c = widen(b);
     const double e = sub(__hiloint2double(0x43300000, (b >> 23) - 127), 4503599627370496.);
@@ -198,7 +204,7 @@ __device__ __forceinline__ void defl64(const lt_nie64 &h, const Nie64 &n, double
         qv = TYPE == 8 ? lo : mul(lo, add(add(n.pt, h.q2st), kv));
     }
     au = mul(h.Ak, atan_quot(nu, du));
-    av = mul(h.hAk, copysign(log1p_quot(add(nv, nv), qv), n.v)); /* hAk < 0: a halo of negative mass */
+    av = flip(mul(h.hAk, log1p_quot(add(nv, nv), qv)), n.v); /* hAk < 0: a halo of negative mass */
 }
 
 /* Adds one pair's deflection in the sky frame. */
