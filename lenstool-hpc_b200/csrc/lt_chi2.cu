@@ -592,7 +592,7 @@ lt_status lt_delense(lt_context *ctx, const lt_catalog *cat, const lt_frame *fra
     }
     std::lock_guard<std::mutex> lock(ctx->mu);
     cudaSetDevice(ctx->device);
-    const ScratchUse use(ctx);
+    const ScratchUse use(ctx, true, kKeptWorkspace);
     Chi2Buf b;
     lt_status st = chi2_buffers(ctx, nsources, nsources, frame, n, b);
     if (st != LT_OK) return st;
@@ -658,9 +658,9 @@ lt_status lt_chi2_batch_precision(lt_context *ctx, const lt_catalog *const *cats
     for (int i = 0; i < sys->nsystems; i++) total += sys->nimages[i];
     std::lock_guard<std::mutex> lock(ctx->mu);
     cudaSetDevice(ctx->device);
-    const ScratchUse use(ctx);
+    const ScratchUse use(ctx, true, kKeptWorkspace);
     /* groups of models: the sources of all in one launch, grid and delensing of each in turn on the
-     * same planes, the links of all in one launch; their results read once a group */
+     * same planes, the links of all in one launch; their results read once a group. */
     const int group = nmodels < kModels ? nmodels : kModels;
     Chi2Buf b;
     st = chi2_buffers(ctx, sys->nsystems, total, frame, n, b, group);

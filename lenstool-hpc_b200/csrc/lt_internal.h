@@ -19,8 +19,8 @@ struct lt_context {
     std::mutex mu;
     std::string last_error;
     /* workspace of the calls that return when their work is done (host-output planes, chi2),
-     * kept from call to call; dev_alloc gives it back when the budget or the device runs out and
-     * no call is in it (scratch_busy) */
+     * kept from call to call (a chi2 adds no more than kKeptWorkspace); dev_alloc gives it back
+     * when the budget or the device runs out and no call is in it (scratch_busy) */
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
     bool scratch_busy = false;
@@ -103,12 +103,27 @@ lt_status cuda_fail(lt_context *ctx, cudaError_t e, const char *what);
 lt_status dev_alloc(lt_context *ctx, void **p, size_t bytes);
 void dev_free(lt_context *ctx, void *p, size_t bytes);
 lt_status scratch_alloc(lt_context *ctx, size_t bytes);
-/* marks the workspace in use for the rest of the caller's scope (which holds ctx->mu) */
+/* marks the workspace in use for the rest of the caller's scope (which holds ctx->mu); what the
+ * scope grew beyond `keep` bytes is given back at its end */
 struct ScratchUse {
     lt_context *ctx;
-    explicit ScratchUse(lt_context *c, bool use = true) : ctx(c) { ctx->scratch_busy = use; }
-    ~ScratchUse() { ctx->scratch_busy = false; }
+    size_t keep;
+    explicit ScratchUse(lt_context *c, bool use = true, size_t most = (size_t)-1)
+        : ctx(c), keep(most > c->scratch_bytes ? most : c->scratch_bytes)
+    {
+        ctx->scratch_busy = use;
+    }
+    ~ScratchUse()
+    {
+        ctx->scratch_busy = false;
+        if (ctx->scratch_bytes <= keep) return;
+        dev_free(ctx, ctx->scratch, ctx->scratch_bytes);
+        ctx->scratch = nullptr;
+        ctx->scratch_bytes = 0;
+    }
 };
+/* a chi2 on 4096^2 keeps its planes (268 MB); above, an allocation is less than 1% of the grid */
+constexpr size_t kKeptWorkspace = (size_t)512 << 20;
 bool is_device_pointer(const void *p);
 std::vector<lt_chunk> make_chunks(const int32_t *type, int n, int max_chunk, const double *dlsds = nullptr);
 
