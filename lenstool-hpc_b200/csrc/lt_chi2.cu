@@ -660,11 +660,14 @@ lt_status lt_chi2_batch_precision(lt_context *ctx, const lt_catalog *const *cats
     cudaSetDevice(ctx->device);
     const ScratchUse use(ctx, true, kKeptWorkspace);
     /* groups of models: the sources of all in one launch, grid and delensing of each in turn on the
-     * same planes, the links of all in one launch; their results read once a group. */
-    const int group = nmodels < kModels ? nmodels : kModels;
+     * same planes, the links of all in one launch; their results read once a group.  Smaller
+     * groups where memory is short: one model's buffers are all that the call cannot do without */
+    int group = nmodels < kModels ? nmodels : kModels;
     Chi2Buf b;
-    st = chi2_buffers(ctx, sys->nsystems, total, frame, n, b, group);
-    if (st != LT_OK) return st;
+    while ((st = chi2_buffers(ctx, sys->nsystems, total, frame, n, b, group)) != LT_OK) {
+        if (group == 1 || (st != LT_ERR_BUDGET && st != LT_ERR_OUT_OF_MEMORY)) return st;
+        group = (group + 1) / 2;
+    }
     cudaStream_t s = nullptr;
     st = upload_systems(ctx, sys, b, s);
     int err = cudaSuccess;

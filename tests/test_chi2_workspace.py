@@ -1,4 +1,5 @@
-"""The chi2's workspace: it is kept from call to call up to a bound."""
+"""The chi2's workspace: it is kept from call to call up to a bound, and a batch of models asks for no more than one
+model's buffers where memory is short."""
 import numpy as np
 import pytest
 
@@ -27,6 +28,16 @@ def _gpu():
     import torch
     if not torch.cuda.is_available():
         pytest.skip("no GPU")
+
+
+def test_many_models_under_a_small_budget():
+    """64 models of 2000 systems: 78 MB of work and results (1.2 MB a model) beside 5 MB of planes and systems."""
+    models, s = _models(64), _systems(2000)
+    with lt.Context(0) as c:
+        want = c.chi2([c.upload(m) for m in models], FRAME, 512, s)
+    with lt.Context(0, 16 * MB) as c:
+        got = c.chi2([c.upload(m) for m in models], FRAME, 512, s)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
 
 
 @pytest.mark.parametrize("n, kept", [(2048, True), (8000, False)])  # planes of 67 MB and of 1 GB
