@@ -296,6 +296,9 @@ lt_status lt_create(int device, size_t budget, lt_context **out)
         return st;
     }
     cudaMemset(ctx->status, 0, 64);
+    /* a copy from pageable memory may still be on its way when it returns: calls on streams that
+     * do not wait for the default one read the tables and the status block */
+    cudaStreamSynchronize(nullptr);
     if (device < 64) {
         std::lock_guard<std::mutex> lock(g_ctx_mu);
         g_contexts[device]++;
