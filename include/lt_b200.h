@@ -262,9 +262,12 @@ lt_status lt_get_kernel_shape(const lt_context *ctx, int32_t precision, int32_t 
                               int32_t *ctas_per_sm);
 /* The full kernel configuration: besides the shape, the threads per CTA (128 or 256; a
  * tile is 32 x pixels_per_thread columns by threads / 32 rows) and the halo records per
- * shared-memory stage (32, 64 or 128).  Grids too small to fill the SMs run in CTAs of 64
- * or 128 threads whatever the configuration says, with the same planes.  LT_FP32C kernels
- * come in the shapes (pixels, CTAs/SM, threads) = (1|2, 1|2, 256), (1, 2|4, 128), (2, 2|3|4, 128), each with
+ * shared-memory stage (32, 64 or 128).  A configuration that was set here or by
+ * lt_set_kernel_shape holds for grids of every size.  With the default and the autotuned ones,
+ * FP64 grids and two-pixel LT_FP32C grids too small to fill the SMs run in CTAs of 64 or 128
+ * threads, with the same planes.  Shapes are those of the kernels that evaluate every pair: an
+ * FP64 call whose far halos are interpolated has none.  LT_FP32C kernels come in the shapes
+ * (pixels, CTAs/SM, threads) = (1|2, 1|2, 256), (1, 2|4, 128), (2, 2|3|4, 128), each with
  * every stage size; the FP64 kernels in their four 256-thread, 64-record shapes.  An
  * unbuilt configuration is LT_ERR_INVALID_ARGUMENT.  lt_set_kernel_shape keeps 256 threads
  * and 64-record stages. */

@@ -540,7 +540,7 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
     a.mult = mult;
     a.scale = scale;
     a.status = ctx->status;
-    a.plain = plain;
+    a.own_shape = a.every_pair = plain;
     cudaStream_t s = (cudaStream_t)stream;
     const int side = call_side(ctx, cat, op, precision, a);
     /* the kernels of one band of rows (the whole grid for device outputs) */
@@ -625,13 +625,15 @@ lt_status lt::run_grid(lt_context *ctx, const lt_catalog *cat, const lt_grid *g,
 
 int lt::call_side(const lt_context *ctx, const lt_catalog *cat, int op, int precision, const GridArgs &a)
 {
-    if (precision == LT_FP32C || cat->nhalos == 0 || a.plain) return 0;
+    if (precision == LT_FP32C || cat->nhalos == 0 || a.every_pair) return 0;
     if (precision == LT_FP64 && (op & OP_HESS)) op &= ~OP_HESS; /* every pair, in the reference's order */
     return op ? tree_side(cat, op, a.nx, a.ny, a.dx, a.dy, ctx->num_sms) : 0;
 }
 
 int lt::launch_fp64(lt_context *ctx, const lt_catalog *cat, int op, int precision, GridArgs &a, int side, void *stream)
 {
+    const int32_t own = a.own_shape;
+    a.own_shape = own || ctx->shape_set[precision][op & 7];
     if (precision == LT_FP64 && (op & OP_HESS)) {
         /* the Hessian with the reference's rounding sequence; with the potential (its own
          * records and registers) as two launches, each writing its planes */
@@ -646,6 +648,7 @@ int lt::launch_fp64(lt_context *ctx, const lt_catalog *cat, int op, int precisio
         a.kinds[0] = KIND_POT;
         a.out[0] = a.out[pot];
         op = OP_POT;
+        a.own_shape = own || ctx->shape_set[precision][op];
     }
     if (side) return launch_tree64(cat, op, a, side, stream);
     return launch_grid64_tiled(op, a, ctx->num_sms, stream, ctx->shape[precision][op & 7]);
@@ -752,6 +755,7 @@ lt_status lt_set_kernel_shape(lt_context *ctx, int32_t precision, int32_t sums, 
         return LT_ERR_INVALID_ARGUMENT;
     std::lock_guard<std::mutex> lock(ctx->mu);
     ctx->shape[precision][sums] = LT_SHAPE(ppt, cps);
+    ctx->shape_set[precision][sums] = true;
     return LT_OK;
 }
 
@@ -781,6 +785,7 @@ lt_status lt_set_kernel_config(lt_context *ctx, int32_t precision, int32_t sums,
     if (!ctx || !sums_ok(precision, sums) || !config_ok(precision, c)) return LT_ERR_INVALID_ARGUMENT;
     std::lock_guard<std::mutex> lock(ctx->mu);
     ctx->shape[precision][sums] = LT_SHAPE4(c->pixels_per_thread, c->ctas_per_sm, c->threads, c->chunk);
+    ctx->shape_set[precision][sums] = true;
     return LT_OK;
 }
 
@@ -861,6 +866,7 @@ lt_status lt_autotune(lt_context *ctx, const lt_catalog *cat, int32_t precision,
         }
     }
     ctx->shape[precision][sums] = best_shape;
+    if (st == LT_OK) ctx->shape_set[precision][sums] = false;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     {

@@ -42,7 +42,8 @@ struct GridArgs {
     const int32_t *list;
     const int32_t *list_count;
     int32_t list_cap;
-    int32_t plain; /* the configured kernel shape even on a small grid, every pair evaluated */
+    int32_t own_shape;  /* the configured kernel shape even on a small grid */
+    int32_t every_pair; /* no halo interpolated */
 };
 
 /* Kernel shape: pixels per thread (1 or 2), resident CTAs per SM the register budget is

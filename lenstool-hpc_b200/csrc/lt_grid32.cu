@@ -392,7 +392,7 @@ static int launch_pass1(lt_context *ctx, const Fp32cCatalog &fc, int op, C32Args
      * deflection and potential like the Hessian; profiles of types 5 and 8 among the halos shift
      * all columns alike but the last, which loses up to 12% (lens maps 36%) above 4 warps. */
     const double warps = ((A.g.nx + 15) / 16) * (double)((A.g.ny + 3) / 4) / (4. * ctx->num_sms);
-    const bool two = P == 2 && !A.g.plain, lens = op == (OP_HESS | OP_POT);
+    const bool two = P == 2 && !A.g.own_shape && !ctx->shape_set[LT_FP32C][op & 7], lens = op == (OP_HESS | OP_POT);
     if (two && warps <= (lens ? 1.6 : 4.)) {
         kern = small_kernel32(op);
         NT = kSmallThreads;

@@ -224,7 +224,7 @@ static int launch_shape(int shape, const GridArgs &a, int num_sms, cudaStream_t 
 {
     /* a grid of less than two CTAs an SM: CTAs of 64 threads, one pixel each, so that it spreads
      * over all SMs, and (reference-order Hessian) two records a thread at a time */
-    if (!a.plain && (long)((a.nx + 31) / 32) * ((a.ny + 7) / 8) < 2 * num_sms)
+    if (!a.own_shape && (long)((a.nx + 31) / 32) * ((a.ny + 7) / 8) < 2 * num_sms)
         return launch_op<OP, 1, false, 4, kSmallThreads, 2>(a, num_sms, s);
     switch (shape) {
     case LT_SHAPE(1, 1): return launch_op<OP, 1, false, 1>(a, num_sms, s);

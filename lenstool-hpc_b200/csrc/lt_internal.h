@@ -29,6 +29,7 @@ struct lt_context {
     void *list = nullptr;      /* pixel list of the FP32C recomputation pass (+ count) */
     size_t list_bytes = 0;
     int shape[3][8] = {};      /* kernel shape per [precision][sums mask], LT_SHAPE4() */
+    bool shape_set[3][8] = {}; /* set by the caller: small grids keep it too */
     cudaStream_t copy_stream = nullptr; /* host-output calls: band copies overlap the next band */
     cudaStream_t band_stream = nullptr; /* and every second band's kernels */
     /* pass timing (lt_set_pass_timing): CUDA events around the passes of FP32C calls */
