@@ -277,7 +277,8 @@ typedef struct {
 lt_status lt_set_kernel_config(lt_context *ctx, int32_t precision, int32_t sums, const lt_kernel_config *config);
 lt_status lt_get_kernel_config(const lt_context *ctx, int32_t precision, int32_t sums, lt_kernel_config *config);
 /* Time every configuration for (precision, sums) on a grid_n x grid_n grid covering the
- * catalogue and keep the fastest in the context; *best_ms (may be NULL) gets its time.
+ * catalogue, every pair evaluated, and keep the fastest in the context; *best_ms (may be
+ * NULL) gets the time of that grid's call with it, as the grid calls make it.
  * The batches built afterwards take the pixels per thread of the tuned LT_FP32C Hessian
  * shape; their persistent kernel has 256 threads and two CTAs per SM (one where the batch
  * has no more tiles than the GPU SMs). */

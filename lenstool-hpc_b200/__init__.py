@@ -420,7 +420,7 @@ class Context:
 
     def autotune(self, cat, precision="fp32c", sums="lens", grid_n=512):
         """Time every kernel configuration on a grid_n^2 grid over the catalogue; keep the
-        fastest.  Returns (pixels_per_thread, ctas_per_sm, ms); kernel_config() gives the
+        fastest.  Returns (pixels_per_thread, ctas_per_sm, ms of one call); kernel_config() gives the
         threads per CTA and the stage size too."""
         cat = self._cat(cat)
         ms = C.c_double()
