@@ -150,7 +150,10 @@ typedef struct {
  * and the FP32C chunk lists are kept: a halo of the FP32 class whose new parameters need
  * FP64 everywhere is evaluated through its FP64 record, an FP64-class halo stays FP64.  A
  * sample outside a profile's domain makes lt_synchronize report LT_ERR_NONFINITE and
- * leaves that halo unchanged.  Batches holding the handle see the update on their next
+ * leaves that halo unchanged.  The FP64 calls that interpolate far halos choose their tiles by
+ * the last parameters that came from the host: after an update from host arrays their planes
+ * equal a fresh upload's bit for bit; from device arrays they may differ in rounding (1e-13 of
+ * max(|value|, RMS)), and take longer where the halos have moved far.  Batches holding the handle see the update on their next
  * launch; do not update a catalogue that in-flight serving requests use.  Host arrays are
  * staged in a per-catalogue device buffer: successive updates of one catalogue go on one
  * stream.  The reference applies a posterior row on the host
@@ -211,8 +214,8 @@ lt_status lt_bayes_create(lt_context *ctx, const lt_bayes_model *model, int32_t 
  * with the row's sigma and cut, takes the potential-parameter step and packs the records
  * as lt_catalog_update does.  Rows are independent (each starts from the model's state).
  * With host rows the cos/sin of sampled angles are taken on the host, so the records
- * equal an upload of the reference's SoA bit for bit; with device rows they are taken on
- * the device.  Host rows are staged in a per-model device buffer: successive applies of
+ * and the planes equal an upload of the reference's SoA bit for bit; with device rows they are
+ * taken on the device (and tiles are chosen as lt_catalog_update says).  Host rows are staged in a per-model device buffer: successive applies of
  * one model go on one stream.  Replaces the per-sample host update and SoA upload of the
  * reference's map loop (utils/maps/main.cpp:428-470). */
 lt_status lt_bayes_apply(lt_context *ctx, lt_bayes *bayes, const double *rows, int32_t nrows,

@@ -399,19 +399,12 @@ lt_status lt_catalog_upload(lt_context *ctx, const lt_halo_soa *s, lt_catalog **
     cat->nhalos = s->nhalos;
     cat->host_recs.resize(s->nhalos);
     cat->host_types.assign(s->type, s->type + s->nhalos);
-    double lo[2] = {0., 0.}, hi[2] = {0., 0.};
+    HaloSpread spread;
     for (int i = 0; i < s->nhalos; i++) {
         pack_one(s, i, cat->host_recs[i]);
-        const double e = s->ellipticity_potential[i], r = (1. + e) / (1. - e); /* 1/q; SIS: 1/q^2 */
-        cat->sum_iq += s->type[i] == 5 ? std::sqrt(r) : r;
-        cat->sum_iq2 += s->type[i] == 5 ? r : r * r;
-        const double p[2] = {s->position_x[i], s->position_y[i]};
-        for (int k = 0; k < 2; k++) {
-            lo[k] = i ? std::min(lo[k], p[k]) : p[k];
-            hi[k] = i ? std::max(hi[k], p[k]) : p[k];
-        }
+        spread.add(s->type[i], s->position_x[i], s->position_y[i], s->ellipticity_potential[i]);
     }
-    cat->box = (hi[0] - lo[0]) * (hi[1] - lo[1]);
+    spread.store(cat);
     std::vector<lt_chunk> ch = make_chunks(s->type, s->nhalos, LT_CHUNK);
     std::vector<double> w(s->nhalos);
     for (int i = 0; i < s->nhalos; i++) w[i] = cat->host_recs[i].w;

@@ -124,53 +124,68 @@ struct ApplyArgs {
     int32_t *status;
 };
 
+/* Halo h's parameters in a row; trig: cos and sin of the row's angles (NULL: taken here). */
+struct HaloState {
+    double x, y, epot, b0, cs, sn, rc, rcut;
+};
+LT_HD inline HaloState bayes_state(const BayesDev &m, const double *row, const double *trig, int h)
+{
+    HaloState o;
+    o.x = m.x[h];
+    o.y = m.y[h];
+    o.epot = m.epot[h];
+    o.cs = m.cs[h];
+    o.sn = m.sn[h];
+    o.rc = m.rc[h];
+    o.rcut = m.rcut[h];
+    double emass = m.emass[h], vdisp = m.vdisp[h];
+    const int p = m.pf[h];
+    if (p < 0) {
+        /* the halo's free parameters (setbayesmapmodels, :142-188) */
+        for (int q = m.col_off[h]; q < m.col_off[h + 1]; q++) {
+            const int c = m.col_idx[q];
+            const double v = row[c];
+            switch (m.col_field[q]) {
+            case LT_BAYES_X: o.x = v; break;
+            case LT_BAYES_Y: o.y = v; break;
+            case LT_BAYES_EPOT: o.epot = v; break;
+            case LT_BAYES_EMASS: emass = v; break;
+            case LT_BAYES_THETA:
+                if (trig) {
+                    o.cs = trig[2 * m.tslot[c]];
+                    o.sn = trig[2 * m.tslot[c] + 1];
+                } else {
+                    sincos(pk::mul(v, m.dtr), &o.sn, &o.cs);
+                }
+                break;
+            case LT_BAYES_RCORE: o.rc = v; break;
+            case LT_BAYES_VDISP: vdisp = v; break;
+            case LT_BAYES_RCUT: o.rcut = v; break;
+            default: break; /* LT_BAYES_Z: the maps' D_LS/D_OS is set at upload */
+            }
+        }
+    } else if (m.hasmag[h]) {
+        /* potfile scaling relations (setScalingRelations, :1613-1634) */
+        const double sig = m.pot_sigma_col[p] >= 0 ? row[m.pot_sigma_col[p]] : m.pot_sigma[p];
+        const double cut = m.pot_cut_col[p] >= 0 ? row[m.pot_cut_col[p]] : m.pot_cut[p];
+        o.rc = m.rcs[h];
+        vdisp = pk::mul(sig, m.fv[h]);
+        o.rcut = pk::mul(cut, m.fr[h]);
+    }
+    pk::calc_potential_parameter(m.types[h], vdisp, emass, o.epot, o.b0);
+    return o;
+}
+
 __global__ void bayes_apply_kernel(const ApplyArgs a)
 {
     const BayesDev &m = a.m;
     const long total = (long)a.nrows * m.n;
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < total; k += (long)gridDim.x * blockDim.x) {
         const int r = (int)(k / m.n), h = (int)(k % m.n);
-        const double *row = a.rows + (size_t)r * m.ncols;
-        const int t = m.types[h];
-        double x = m.x[h], y = m.y[h], epot = m.epot[h], emass = m.emass[h], cs = m.cs[h], sn = m.sn[h];
-        double rc = m.rc[h], vdisp = m.vdisp[h], rcut = m.rcut[h];
-        const int p = m.pf[h];
-        if (p < 0) {
-            /* the halo's free parameters (setbayesmapmodels, :142-188) */
-            for (int q = m.col_off[h]; q < m.col_off[h + 1]; q++) {
-                const int c = m.col_idx[q];
-                const double v = row[c];
-                switch (m.col_field[q]) {
-                case LT_BAYES_X: x = v; break;
-                case LT_BAYES_Y: y = v; break;
-                case LT_BAYES_EPOT: epot = v; break;
-                case LT_BAYES_EMASS: emass = v; break;
-                case LT_BAYES_THETA:
-                    if (a.trig) {
-                        const double *tc = a.trig + 2 * ((size_t)r * m.ntheta + m.tslot[c]);
-                        cs = tc[0];
-                        sn = tc[1];
-                    } else {
-                        sincos(pk::mul(v, m.dtr), &sn, &cs);
-                    }
-                    break;
-                case LT_BAYES_RCORE: rc = v; break;
-                case LT_BAYES_VDISP: vdisp = v; break;
-                case LT_BAYES_RCUT: rcut = v; break;
-                default: break; /* LT_BAYES_Z: the maps' D_LS/D_OS is set at upload */
-                }
-            }
-        } else if (m.hasmag[h]) {
-            /* potfile scaling relations (setScalingRelations, :1613-1634) */
-            const double sig = m.pot_sigma_col[p] >= 0 ? row[m.pot_sigma_col[p]] : m.pot_sigma[p];
-            const double cut = m.pot_cut_col[p] >= 0 ? row[m.pot_cut_col[p]] : m.pot_cut[p];
-            rc = m.rcs[h];
-            vdisp = pk::mul(sig, m.fv[h]);
-            rcut = pk::mul(cut, m.fr[h]);
-        }
-        double b0;
-        pk::calc_potential_parameter(t, vdisp, emass, epot, b0);
-        if (!store_records(a.cats[r], h, t, x, y, cs, sn, b0, epot, rc, rcut)) flag(a.status, (int32_t)LT_ERR_NONFINITE);
+        const HaloState o = bayes_state(m, a.rows + (size_t)r * m.ncols,
+                                        a.trig ? a.trig + 2 * (size_t)r * m.ntheta : nullptr, h);
+        if (!store_records(a.cats[r], h, m.types[h], o.x, o.y, o.cs, o.sn, o.b0, o.epot, o.rc, o.rcut))
+            flag(a.status, (int32_t)LT_ERR_NONFINITE);
     }
 }
 
@@ -186,6 +201,10 @@ struct lt_bayes {
     void *mem = nullptr;
     size_t bytes = 0;
     BayesDev dev;
+    std::vector<unsigned char> image; /* the host's copy of mem */
+    BayesDev host;                    /* dev with its pointers into it */
+    std::vector<double> epot;         /* the model's ellipticity_potential after its last step */
+    std::vector<char> moves;          /* per halo: a column sets its position or ellipticity */
     void *stage = nullptr;
     size_t stage_bytes = 0;
 };
@@ -278,6 +297,20 @@ extern "C" lt_status lt_catalog_update(lt_context *ctx, lt_catalog *cat, const l
     count_launch(1);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "catalogue update");
+    if (!device) {
+        bool known = true;
+        for (int k = 0; k < 7; k++) known &= !is_device_pointer(in[k]);
+        HaloSpread spread;
+        for (int i = 0; known && i < cat->nhalos; i++) {
+            const int t = cat->host_types[i];
+            double b0, eps;
+            pk::potential_parameters(t, p->vdisp[i], p->ellipticity[i], b0, eps);
+            known = p->ellipticity[i] >= 0. && p->ellipticity[i] < 1. && std::isfinite(p->ellipticity_angle[i]) &&
+                    pk::record_ok(t, p->position_x[i], p->position_y[i], b0, 1., 0., eps, p->rcore[i], p->rcut[i]);
+            spread.add(t, p->position_x[i], p->position_y[i], eps);
+        }
+        if (known) spread.store(cat); /* a sample with a halo outside its domain: as it was */
+    }
     return LT_OK;
 }
 
@@ -364,9 +397,11 @@ extern "C" lt_status lt_bayes_create(lt_context *ctx, const lt_bayes_model *mode
     for (int i = 0; i < n; i++) count[i + 1] += count[i];
     const int nused = n ? count[n] : 0;
     std::vector<int32_t> col_idx((size_t)nused), col_field((size_t)nused), fill(count.begin(), count.end());
+    std::vector<char> moves((size_t)n, 0);
     for (int c = 0; c < ncolumns; c++) {
         const int f = columns[c].field;
         if (f < LT_BAYES_X || f > LT_BAYES_Z) continue;
+        if (f <= LT_BAYES_EMASS) moves[columns[c].target] = 1;
         const int q = fill[columns[c].target]++;
         col_idx[q] = c;
         col_field[q] = f;
@@ -401,14 +436,20 @@ extern "C" lt_status lt_bayes_create(lt_context *ctx, const lt_bayes_model *mode
     b->npot = npotfiles;
     b->types.assign(model->type, model->type + n);
     b->theta_cols = theta_cols;
+    b->moves = moves;
+    b->epot = base[2];
+    for (int i = 0; i < n; i++) {
+        double emass = base[3][i], b0;
+        pk::calc_potential_parameter(model->type[i], model->vdisp[i], emass, b->epot[i], b0);
+    }
     b->dtr = acos(-1.) / 180.;
     /* one allocation: doubles, then int32 arrays */
     const size_t nd = 12 * (size_t)n + 2 * (size_t)npotfiles;
     const size_t ni = 5 * (size_t)n + 1 + 2 * (size_t)nused + (size_t)ncolumns + 2 * (size_t)npotfiles;
     b->bytes = nd * sizeof(double) + ni * sizeof(int32_t) + 16;
-    std::vector<unsigned char> host(b->bytes, 0);
-    double *hd = (double *)host.data();
-    int32_t *hi = (int32_t *)(host.data() + nd * sizeof(double));
+    b->image.assign(b->bytes, 0);
+    double *hd = (double *)b->image.data();
+    int32_t *hi = (int32_t *)(b->image.data() + nd * sizeof(double));
     std::lock_guard<std::mutex> lock(ctx->mu);
     cudaSetDevice(ctx->device);
     lt_status st = dev_alloc(ctx, &b->mem, b->bytes);
@@ -419,47 +460,47 @@ extern "C" lt_status lt_bayes_create(lt_context *ctx, const lt_bayes_model *mode
     double *dd = (double *)b->mem;
     int32_t *di = (int32_t *)((char *)b->mem + nd * sizeof(double));
     size_t od = 0, oi = 0;
-    auto put_d = [&](const double *src, size_t cnt) {
+    BayesDev &m = b->dev, &w = b->host;
+    auto put_d = [&](const double *BayesDev::*field, const double *src, size_t cnt) {
         if (cnt) memcpy(hd + od, src, cnt * sizeof(double));
-        const double *d = dd + od;
+        m.*field = dd + od;
+        w.*field = hd + od;
         od += cnt;
-        return d;
     };
-    auto put_i = [&](const int32_t *src, size_t cnt) {
+    auto put_i = [&](const int32_t *BayesDev::*field, const int32_t *src, size_t cnt) {
         if (cnt) memcpy(hi + oi, src, cnt * sizeof(int32_t));
-        const int32_t *d = di + oi;
+        m.*field = di + oi;
+        w.*field = hi + oi;
         oi += cnt;
-        return d;
     };
-    BayesDev &m = b->dev;
-    m.n = n;
-    m.ncols = ncolumns;
-    m.ntheta = (int)theta_cols.size();
-    m.dtr = b->dtr;
-    m.x = put_d(base[0].data(), n);
-    m.y = put_d(base[1].data(), n);
-    m.epot = put_d(base[2].data(), n);
-    m.emass = put_d(base[3].data(), n);
-    m.cs = put_d(base[4].data(), n);
-    m.sn = put_d(base[5].data(), n);
-    m.rc = put_d(base[6].data(), n);
-    m.vdisp = put_d(base[7].data(), n);
-    m.rcut = put_d(base[8].data(), n);
-    m.fv = put_d(fv.data(), n);
-    m.fr = put_d(fr.data(), n);
-    m.rcs = put_d(rcs.data(), n);
-    m.pot_sigma = put_d(pot_sigma.data(), npotfiles);
-    m.pot_cut = put_d(pot_cut.data(), npotfiles);
-    m.types = put_i(model->type, n);
-    m.pf = put_i(pf.data(), n);
-    m.hasmag = put_i(hasmag.data(), n);
-    m.col_off = put_i(count.data(), (size_t)n + 1);
-    m.col_idx = put_i(col_idx.data(), nused);
-    m.col_field = put_i(col_field.data(), nused);
-    m.tslot = put_i(tslot.data(), ncolumns);
-    m.pot_sigma_col = put_i(pot_sigma_col.data(), npotfiles);
-    m.pot_cut_col = put_i(pot_cut_col.data(), npotfiles);
-    const cudaError_t e = cudaMemcpy(b->mem, host.data(), b->bytes, cudaMemcpyHostToDevice);
+    m.n = w.n = n;
+    m.ncols = w.ncols = ncolumns;
+    m.ntheta = w.ntheta = (int)theta_cols.size();
+    m.dtr = w.dtr = b->dtr;
+    put_d(&BayesDev::x, base[0].data(), n);
+    put_d(&BayesDev::y, base[1].data(), n);
+    put_d(&BayesDev::epot, base[2].data(), n);
+    put_d(&BayesDev::emass, base[3].data(), n);
+    put_d(&BayesDev::cs, base[4].data(), n);
+    put_d(&BayesDev::sn, base[5].data(), n);
+    put_d(&BayesDev::rc, base[6].data(), n);
+    put_d(&BayesDev::vdisp, base[7].data(), n);
+    put_d(&BayesDev::rcut, base[8].data(), n);
+    put_d(&BayesDev::fv, fv.data(), n);
+    put_d(&BayesDev::fr, fr.data(), n);
+    put_d(&BayesDev::rcs, rcs.data(), n);
+    put_d(&BayesDev::pot_sigma, pot_sigma.data(), npotfiles);
+    put_d(&BayesDev::pot_cut, pot_cut.data(), npotfiles);
+    put_i(&BayesDev::types, model->type, n);
+    put_i(&BayesDev::pf, pf.data(), n);
+    put_i(&BayesDev::hasmag, hasmag.data(), n);
+    put_i(&BayesDev::col_off, count.data(), (size_t)n + 1);
+    put_i(&BayesDev::col_idx, col_idx.data(), nused);
+    put_i(&BayesDev::col_field, col_field.data(), nused);
+    put_i(&BayesDev::tslot, tslot.data(), ncolumns);
+    put_i(&BayesDev::pot_sigma_col, pot_sigma_col.data(), npotfiles);
+    put_i(&BayesDev::pot_cut_col, pot_cut_col.data(), npotfiles);
+    const cudaError_t e = cudaMemcpy(b->mem, b->image.data(), b->bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         dev_free(ctx, b->mem, b->bytes);
         delete b;
@@ -522,6 +563,23 @@ extern "C" lt_status lt_bayes_apply(lt_context *ctx, lt_bayes *b, const double *
     count_launch(1);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "bayes rows");
+    for (int r = 0; !dev_rows && r < nrows; r++) {
+        HaloSpread spread;
+        bool known = true;
+        for (int h = 0; known && h < b->n; h++) {
+            double x = b->host.x[h], y = b->host.y[h], epot = b->epot[h];
+            if (b->moves[h]) {
+                const HaloState o = bayes_state(b->host, rows + (size_t)r * b->ncols,
+                                                (const double *)(host.data() + o_trig) + 2 * (size_t)r * ntheta, h);
+                x = o.x;
+                y = o.y;
+                epot = o.epot;
+            }
+            known = std::isfinite(x) && std::isfinite(y) && epot >= 0. && epot < 1.;
+            spread.add(b->types[h], x, y, epot);
+        }
+        if (known) spread.store(cats[r]);
+    }
     return LT_OK;
 }
 

@@ -2,6 +2,7 @@
  * lt_internal.h -- library-internal declarations shared by the C-ABI translation units.
  */
 #pragma once
+#include <cmath>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -47,8 +48,7 @@ struct lt_catalog {
     size_t bytes = 0;
     std::vector<lt_rec64> host_recs;     /* packed records, host copy */
     std::vector<int32_t> host_types;     /* profile type per halo */
-    double sum_iq = 0, sum_iq2 = 0, box = 0; /* sums of 1/q and 1/q^2 over the halos, area of their
-                                            bounding box, at upload (tree_side's estimate) */
+    double sum_iq = 0, sum_iq2 = 0, box = 0; /* HaloSpread of the last parameters known to the host */
     void *aux = nullptr;                 /* FP32C records and chunks, device */
     size_t aux_bytes = 0;
     void *stage = nullptr;               /* device staging of host parameters (lt_catalog_update) */
@@ -78,6 +78,32 @@ struct Fp32cCatalog {
     int32_t *idx32;  /* per halo: its FP32 record, or -1 for an FP64-class halo (device) */
     int32_t *types;  /* per halo profile type (device) */
     lt_nie64 *nie;   /* per halo (upload order): the FP64 closed-form record */
+};
+
+/* What tree_side() chooses a tile by: the sums of 1/q and 1/q^2 over the halos and the area of their
+ * bounding box.  Uploads and updates from host values add the halos in the catalogue's order, so
+ * that equal parameters choose alike and give the same planes. */
+struct HaloSpread {
+    double iq = 0., iq2 = 0., lo[2] = {0., 0.}, hi[2] = {0., 0.};
+    bool first = true;
+    void add(int type, double x, double y, double epot)
+    {
+        const double r = (1. + epot) / (1. - epot); /* 1/q; SIS: 1/q^2 */
+        iq += type == 5 ? std::sqrt(r) : r;
+        iq2 += type == 5 ? r : r * r;
+        const double p[2] = {x, y};
+        for (int k = 0; k < 2; k++) {
+            lo[k] = first || p[k] < lo[k] ? p[k] : lo[k];
+            hi[k] = first || p[k] > hi[k] ? p[k] : hi[k];
+        }
+        first = false;
+    }
+    void store(lt_catalog *cat) const
+    {
+        cat->sum_iq = iq;
+        cat->sum_iq2 = iq2;
+        cat->box = (hi[0] - lo[0]) * (hi[1] - lo[1]);
+    }
 };
 
 /* the closed-form records of a catalogue (device) */
