@@ -399,12 +399,12 @@ lt_status lt_catalog_upload(lt_context *ctx, const lt_halo_soa *s, lt_catalog **
     cat->nhalos = s->nhalos;
     cat->host_recs.resize(s->nhalos);
     cat->host_types.assign(s->type, s->type + s->nhalos);
-    HaloSpread spread;
-    for (int i = 0; i < s->nhalos; i++) {
-        pack_one(s, i, cat->host_recs[i]);
-        spread.add(s->type[i], s->position_x[i], s->position_y[i], s->ellipticity_potential[i]);
-    }
-    spread.store(cat);
+    for (int i = 0; i < s->nhalos; i++) pack_one(s, i, cat->host_recs[i]);
+    halo_spread(s->nhalos, [&](int, int i, int end) {
+        HaloSpread b;
+        for (; i < end; i++) b.add(s->type[i], s->position_x[i], s->position_y[i], s->ellipticity_potential[i]);
+        return b;
+    }).store(cat);
     std::vector<lt_chunk> ch = make_chunks(s->type, s->nhalos, LT_CHUNK);
     std::vector<double> w(s->nhalos);
     for (int i = 0; i < s->nhalos; i++) w[i] = cat->host_recs[i].w;

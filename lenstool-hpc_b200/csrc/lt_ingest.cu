@@ -203,8 +203,8 @@ struct lt_bayes {
     BayesDev dev;
     std::vector<unsigned char> image; /* the host's copy of mem */
     BayesDev host;                    /* dev with its pointers into it */
-    std::vector<double> epot;         /* the model's ellipticity_potential after its last step */
-    std::vector<char> moves;          /* per halo: a column sets its position or ellipticity */
+    std::vector<HaloSpread> spread;   /* the model's, block by block */
+    std::vector<char> moves;          /* per block: a column sets a position or an ellipticity */
     void *stage = nullptr;
     size_t stage_bytes = 0;
 };
@@ -218,6 +218,18 @@ static lt_status grow(lt_context *ctx, void **p, size_t *have, size_t need)
     lt_status st = dev_alloc(ctx, p, need);
     if (st == LT_OK) *have = need;
     return st;
+}
+
+/* The spread of halos h .. end - 1 in a row; `known` false if one is outside its domain. */
+static HaloSpread row_block(const lt_bayes *b, const double *row, const double *trig, int h, int end, bool &known)
+{
+    HaloSpread s;
+    for (; h < end; h++) {
+        const HaloState o = bayes_state(b->host, row, trig, h);
+        known &= std::isfinite(o.x) && std::isfinite(o.y) && o.epot >= 0. && o.epot < 1.;
+        s.add(b->types[h], o.x, o.y, o.epot);
+    }
+    return s;
 }
 
 static bool same_types(const lt_catalog *cat, const std::vector<int32_t> &types)
@@ -300,15 +312,18 @@ extern "C" lt_status lt_catalog_update(lt_context *ctx, lt_catalog *cat, const l
     if (!device) {
         bool known = true;
         for (int k = 0; k < 7; k++) known &= !is_device_pointer(in[k]);
-        HaloSpread spread;
-        for (int i = 0; known && i < cat->nhalos; i++) {
-            const int t = cat->host_types[i];
-            double b0, eps;
-            pk::potential_parameters(t, p->vdisp[i], p->ellipticity[i], b0, eps);
-            known = p->ellipticity[i] >= 0. && p->ellipticity[i] < 1. && std::isfinite(p->ellipticity_angle[i]) &&
-                    pk::record_ok(t, p->position_x[i], p->position_y[i], b0, 1., 0., eps, p->rcore[i], p->rcut[i]);
-            spread.add(t, p->position_x[i], p->position_y[i], eps);
-        }
+        const HaloSpread spread = halo_spread(known ? cat->nhalos : 0, [&](int, int i, int end) {
+            HaloSpread b;
+            for (; i < end; i++) {
+                const int t = cat->host_types[i];
+                double b0, eps;
+                pk::potential_parameters(t, p->vdisp[i], p->ellipticity[i], b0, eps);
+                known &= p->ellipticity[i] >= 0. && p->ellipticity[i] < 1. && std::isfinite(p->ellipticity_angle[i]) &&
+                         pk::record_ok(t, p->position_x[i], p->position_y[i], b0, 1., 0., eps, p->rcore[i], p->rcut[i]);
+                b.add(t, p->position_x[i], p->position_y[i], eps);
+            }
+            return b;
+        });
         if (known) spread.store(cat); /* a sample with a halo outside its domain: as it was */
     }
     return LT_OK;
@@ -397,11 +412,11 @@ extern "C" lt_status lt_bayes_create(lt_context *ctx, const lt_bayes_model *mode
     for (int i = 0; i < n; i++) count[i + 1] += count[i];
     const int nused = n ? count[n] : 0;
     std::vector<int32_t> col_idx((size_t)nused), col_field((size_t)nused), fill(count.begin(), count.end());
-    std::vector<char> moves((size_t)n, 0);
+    std::vector<char> moves((size_t)n / kSpreadBlock + 1, 0);
     for (int c = 0; c < ncolumns; c++) {
         const int f = columns[c].field;
         if (f < LT_BAYES_X || f > LT_BAYES_Z) continue;
-        if (f <= LT_BAYES_EMASS) moves[columns[c].target] = 1;
+        if (f <= LT_BAYES_EMASS) moves[columns[c].target / kSpreadBlock] = 1;
         const int q = fill[columns[c].target]++;
         col_idx[q] = c;
         col_field[q] = f;
@@ -437,11 +452,6 @@ extern "C" lt_status lt_bayes_create(lt_context *ctx, const lt_bayes_model *mode
     b->types.assign(model->type, model->type + n);
     b->theta_cols = theta_cols;
     b->moves = moves;
-    b->epot = base[2];
-    for (int i = 0; i < n; i++) {
-        double emass = base[3][i], b0;
-        pk::calc_potential_parameter(model->type[i], model->vdisp[i], emass, b->epot[i], b0);
-    }
     b->dtr = acos(-1.) / 180.;
     /* one allocation: doubles, then int32 arrays */
     const size_t nd = 12 * (size_t)n + 2 * (size_t)npotfiles;
@@ -500,6 +510,15 @@ extern "C" lt_status lt_bayes_create(lt_context *ctx, const lt_bayes_model *mode
     put_i(&BayesDev::tslot, tslot.data(), ncolumns);
     put_i(&BayesDev::pot_sigma_col, pot_sigma_col.data(), npotfiles);
     put_i(&BayesDev::pot_cut_col, pot_cut_col.data(), npotfiles);
+    for (int i = 0; i < n; i += kSpreadBlock) {
+        HaloSpread s;
+        for (int h = i; h < n && h < i + kSpreadBlock; h++) {
+            double epot = w.epot[h], emass = w.emass[h], b0;
+            pk::calc_potential_parameter(w.types[h], w.vdisp[h], emass, epot, b0);
+            s.add(w.types[h], w.x[h], w.y[h], epot);
+        }
+        b->spread.push_back(s);
+    }
     const cudaError_t e = cudaMemcpy(b->mem, b->image.data(), b->bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         dev_free(ctx, b->mem, b->bytes);
@@ -564,20 +583,11 @@ extern "C" lt_status lt_bayes_apply(lt_context *ctx, lt_bayes *b, const double *
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "bayes rows");
     for (int r = 0; !dev_rows && r < nrows; r++) {
-        HaloSpread spread;
         bool known = true;
-        for (int h = 0; known && h < b->n; h++) {
-            double x = b->host.x[h], y = b->host.y[h], epot = b->epot[h];
-            if (b->moves[h]) {
-                const HaloState o = bayes_state(b->host, rows + (size_t)r * b->ncols,
-                                                (const double *)(host.data() + o_trig) + 2 * (size_t)r * ntheta, h);
-                x = o.x;
-                y = o.y;
-                epot = o.epot;
-            }
-            known = std::isfinite(x) && std::isfinite(y) && epot >= 0. && epot < 1.;
-            spread.add(b->types[h], x, y, epot);
-        }
+        const HaloSpread spread = halo_spread(b->n, [&](int k, int h, int end) {
+            const double *trig = (const double *)(host.data() + o_trig) + 2 * (size_t)r * ntheta;
+            return b->moves[k] ? row_block(b, rows + (size_t)r * b->ncols, trig, h, end, known) : b->spread[k];
+        });
         if (known) spread.store(cats[r]);
     }
     return LT_OK;

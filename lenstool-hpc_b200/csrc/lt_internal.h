@@ -81,30 +81,46 @@ struct Fp32cCatalog {
 };
 
 /* What tree_side() chooses a tile by: the sums of 1/q and 1/q^2 over the halos and the area of their
- * bounding box.  Uploads and updates from host values add the halos in the catalogue's order, so
- * that equal parameters choose alike and give the same planes. */
+ * bounding box.  Uploads and updates from host values add blocks of kSpreadBlock halos in the
+ * catalogue's order, so that equal parameters choose alike and give the same planes, and rows that
+ * move a few halos add up those blocks alone. */
+constexpr int kSpreadBlock = 32;
 struct HaloSpread {
-    double iq = 0., iq2 = 0., lo[2] = {0., 0.}, hi[2] = {0., 0.};
-    bool first = true;
+    double iq = 0., iq2 = 0., lo[2] = {INFINITY, INFINITY}, hi[2] = {-INFINITY, -INFINITY};
     void add(int type, double x, double y, double epot)
     {
         const double r = (1. + epot) / (1. - epot); /* 1/q; SIS: 1/q^2 */
-        iq += type == 5 ? std::sqrt(r) : r;
-        iq2 += type == 5 ? r : r * r;
-        const double p[2] = {x, y};
+        HaloSpread h;
+        h.iq = type == 5 ? std::sqrt(r) : r;
+        h.iq2 = type == 5 ? r : r * r;
+        h.lo[0] = h.hi[0] = x;
+        h.lo[1] = h.hi[1] = y;
+        add(h);
+    }
+    void add(const HaloSpread &o)
+    {
+        iq += o.iq;
+        iq2 += o.iq2;
         for (int k = 0; k < 2; k++) {
-            lo[k] = first || p[k] < lo[k] ? p[k] : lo[k];
-            hi[k] = first || p[k] > hi[k] ? p[k] : hi[k];
+            lo[k] = o.lo[k] < lo[k] ? o.lo[k] : lo[k];
+            hi[k] = o.hi[k] > hi[k] ? o.hi[k] : hi[k];
         }
-        first = false;
     }
     void store(lt_catalog *cat) const
     {
         cat->sum_iq = iq;
         cat->sum_iq2 = iq2;
-        cat->box = (hi[0] - lo[0]) * (hi[1] - lo[1]);
+        cat->box = hi[0] > lo[0] && hi[1] > lo[1] ? (hi[0] - lo[0]) * (hi[1] - lo[1]) : 0.;
     }
 };
+/* The spread of halos 0 .. n - 1; block(b, i0, i1) gives that of one block of them. */
+template <class Block>
+HaloSpread halo_spread(int n, Block block)
+{
+    HaloSpread s;
+    for (int i = 0; i < n; i += kSpreadBlock) s.add(block(i / kSpreadBlock, i, i + kSpreadBlock < n ? i + kSpreadBlock : n));
+    return s;
+}
 
 /* the closed-form records of a catalogue (device) */
 inline const lt_nie64 *nie_of(const lt_catalog *cat)
