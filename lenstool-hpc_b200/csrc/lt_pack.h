@@ -242,13 +242,15 @@ LT_HD inline void pack_nie64(const lt_rec64 &r, int type, lt_nie64 &o)
     const double t05 = (type == 81) ? div(rcut, sub(rcut, r.rc)) : 1.0;
     const double K = mul(0.5, mul(mul(r.b0, ome), t05));
     const double sc = mul(ope, r.rc), st = mul(ope, rcut);
-    const double sc2 = mul(sc, sc), st2 = mul(st, st), ds2 = mul(sub(sc, st), add(sc, st));
+    /* radii close to each other: rc - rcut is exact, the difference of two rounded products is not */
+    const double ds = rcut < mul(2., r.rc) ? mul(ope, sub(r.rc, rcut)) : sub(sc, st);
+    const double sc2 = mul(sc, sc), st2 = mul(st, st), ds2 = mul(ds, add(sc, st));
     const double c1 = sub(q2, 1.);
     o.q2 = q2;
     o.k = div(mul(2., sqr(e)), ope);
     o.sc = sc;
     o.st = st;
-    o.ds = sub(sc, st);
+    o.ds = ds;
     o.q2sc2 = mul(q2, sc2);
     o.q2st2 = mul(q2, st2);
     o.dq2s2 = mul(q2, ds2);
@@ -260,7 +262,7 @@ LT_HD inline void pack_nie64(const lt_rec64 &r, int type, lt_nie64 &o)
     o.K = K;
     o.Kc1sc2 = mul(mul(K, c1), sc2);
     o.Kc1st2 = mul(mul(K, c1), st2);
-    o.dsq2 = mul(q2, sub(sc, st));
+    o.dsq2 = mul(q2, ds);
     o.q2sc = mul(q2, sc);
     o.q2st = mul(q2, st);
     o.qsc = mul(q, sc);
