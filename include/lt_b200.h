@@ -330,9 +330,10 @@ lt_status lt_batch_create(lt_context *ctx, const lt_request *reqs, int32_t nreqs
 /* Replay the batch's graph on `stream` (asynchronous; lt_synchronize reports errors). */
 lt_status lt_batch_launch(lt_context *ctx, lt_batch *batch, void *stream);
 int32_t lt_batch_size(const lt_batch *batch);
-/* The batch's kernel configuration: its persistent kernel's pixels per thread and CTAs
- * per SM for LT_FP32C tiles (taken at lt_batch_create from the context's LT_FP32C Hessian
- * shape, as lt_autotune left it), 256 threads, 64-record stages. */
+/* The batch's kernel configuration: its persistent kernel's pixels per thread for LT_FP32C
+ * tiles (taken at lt_batch_create from the context's LT_FP32C Hessian shape, as lt_autotune
+ * left it), the CTAs per SM (two; one where the batch has no more tiles than the GPU SMs),
+ * 256 threads, 64-record stages. */
 lt_status lt_batch_config(const lt_batch *batch, lt_kernel_config *config);
 lt_status lt_batch_destroy(lt_context *ctx, lt_batch *batch);
 

@@ -389,8 +389,9 @@ static int launch_pass1(lt_context *ctx, const Fp32cCatalog &fc, int op, C32Args
      *   16.9     587 / 488 / 512                    1097 / 1027 / 1105
      *   26.2     821 / 768 / 770                    1537 / 1614 / 1630
      *   32.0    1048 / 918 / 935                    1959 / 1932 / 1994
-     * deflection and potential like the Hessian; profiles of types 5 and 8 among the halos shift
-     * all columns alike but the last, which loses up to 12% (lens maps 36%) above 4 warps. */
+     * deflection and potential like the Hessian.  Profiles of types 5 and 8 among the halos shift
+     * all columns alike but the last: 64 x 2 loses up to 12% (lens maps 36%) to the others above 4
+     * warps, where it is not taken. */
     const double warps = ((A.g.nx + 15) / 16) * (double)((A.g.ny + 3) / 4) / (4. * ctx->num_sms);
     const bool two = P == 2 && !A.g.own_shape && !ctx->shape_set[LT_FP32C][op & 7], lens = op == (OP_HESS | OP_POT);
     if (two && warps <= (lens ? 1.6 : 4.)) {

@@ -186,7 +186,7 @@ __device__ __forceinline__ Mat mdci05(double x, double y, double eps, double rc,
  *     RN(1/w), unless w's significand is all ones (x's then ends in 11..10 or 11..11).
  * tests/test_hess_exact.py repeats these steps on every operand of small precisions.  The
  * operands they do not cover (those, and values near the ends of the exponent range, where a
- * remainder is not exact) are found by `odd_operand` and go through mdci05. */
+ * remainder is not exact) are found by `Odd` and go through mdci05. */
 __device__ __forceinline__ double quot(double a, double b, double y)
 {
     const double q = M(a, y);

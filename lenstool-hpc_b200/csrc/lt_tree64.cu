@@ -17,11 +17,16 @@
  * rho^-16 with rho the sum of the semi-axes of the largest regular ellipse around the tile, so a
  * halo is far when
  *   q^2 (max(0, d - diagonal/2)^2 + s^2) >= (kFar h)^2,
- * d from the tile's centre, h the larger half width, and lies outside the circle around the tile.  kFar is taken per sum from the measured
- * error of one term against extended precision (q 0.4 to 0.9, random orientation, core and cut
- * radii; relative to the term): deflection 5e-15 at 3.2, potential 2e-16 at 3.0, convergence and
- * shear 3e-15 at 4.0.  A far term is ~1% of its sum, so the truncation stays below the sum's own
- * rounding.
+ * d from the tile's centre, h the larger half width, and lies outside the circle around the tile.
+ * kFar is 3.2 for the deflection, 3.0 for the potential, 4.0 for convergence and shear.  The largest
+ * truncation of one term at that limit against extended precision (q 0.02 to 1, random
+ * orientation, core and cut radii; relative to its largest value over the tile): PIEMD 5e-15,
+ * 3e-15, 4e-15; cut dPIE 7e-15, 1.4e-15, 7e-15 up to q = 0.9 and 2.7e-14, 2.5e-15, 2.0e-14 for
+ * rounder ones, beyond whose cut core and cut terms cancel; SIS 1.1e-14, 1.1e-15, 4.5e-15 down to
+ * q = 0.7 and 7e-14, 6e-15, 9e-15 at 0.02.  It falls by 16 powers of the distance, so that in a map
+ * the sums' rounding is the larger: deflection of 200 halos on 1024^2 3.5e-16 (2-norm) of extended
+ * precision, every pair in turn in 64 bits 5.4e-16 to 5.8e-16; fields with one dominant halo of
+ * any of these kinds 2e-16 to 1.1e-15, at single pixels up to 4e-14 of the RMS.
  *
  * Layout.  One CTA of 256 threads a tile, a cluster of four CTAs a parent (two and eight for a
  * grid of few tiles: half of the tile's far halos and of its passes each).  A CTA sorts the
@@ -34,7 +39,7 @@
  * Bound by the FP64 pipe and, with few tiles, by the dearest tile's chain, so rows of parents
  * start from the middle of the grid outwards, where most halos are.
  * B200, ms, tiles alone (no parent, tiles streamed in order) / middle first and two records at a
- * time / parents: deflection of 200 halos on 1024^2 0.375 / 0.340 / 0.223, of 1000 on 4096^2
+ * time / parents: deflection of 200 halos on 1024^2 0.375 / 0.340 / 0.225, of 1000 on 4096^2
  * 6.6 / 5.03 / 3.27; potential of 200 on 512^2 0.24 / 0.25 / 0.18; lens maps of 500 on 1199 x 901
  * 1.69 / 1.56 / 1.01.
  */
