@@ -666,6 +666,7 @@ lt_status lt_chi2_batch_precision(lt_context *ctx, const lt_catalog *const *cats
     Chi2Buf b;
     while ((st = chi2_buffers(ctx, sys->nsystems, total, frame, n, b, group)) != LT_OK) {
         if (group == 1 || (st != LT_ERR_BUDGET && st != LT_ERR_OUT_OF_MEMORY)) return st;
+        cudaGetLastError(); /* of a refused allocation: not the launches' */
         group = (group + 1) / 2;
     }
     cudaStream_t s = nullptr;
