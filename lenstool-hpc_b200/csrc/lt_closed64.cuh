@@ -92,7 +92,7 @@ __device__ __forceinline__ double widen(int bits) { return __hiloint2double((bit
  *   atan a = atan c + atan t,  t = (min - c max)/(max + c min),  |t| <= 1/128,
  * and atan t = t - t^3/3 + t^5/5 - t^7/7 (truncation t^9/9 < 2e-18 of t).  One reciprocal,
  * 12 FP64 operations; within 2 ulp of atan(n/d) while the larger of |n| and d is within FP32's
- * range (lengths of 1e-19 to 1e19 arcsec; longer cut radii do not enter, pack_nie64).  j = 0
+ * range (pack_nie64 sees to it that radii far outside the field's scales do not leave it).  j = 0
  * leaves t = a exactly, so small quotients keep their relative accuracy. */
 __device__ __forceinline__ double atan_quot(double n, double d)
 {
@@ -101,7 +101,7 @@ __device__ __forceinline__ double atan_quot(double n, double d)
     const float nf = __double2float_rn(an), df = __double2float_rn(d);
     const bool swap = nf > df;
     const double mn = swap ? d : an, mx = swap ? an : d;
-    const float af = __saturatef(__fmul_rn(fminf(nf, df), frcp(fmaxf(nf, df)))); /* 0/0 (below 2^-126): 0 */
+    const float af = fminf(__fmul_rn(fminf(nf, df), frcp(fmaxf(nf, df))), 1.f);
     const float jf = __fmaf_rn(af, 64.f, 12582912.f); /* 1.5 x 2^23 + j */
     const int j = __float_as_int(jf) & 127;
     const double c = j ? widen(__float_as_int(__fmul_rn(__fsub_rn(jf, 12582912.f), 0.015625f))) : 0.;
@@ -121,7 +121,7 @@ __device__ __forceinline__ double atan_quot(double n, double d)
 __device__ __forceinline__ double log1p_quot(double n, double d)
 {
     using namespace c64;
-    const float m = fmaxf(__fmaf_rn(__double2float_rn(n), frcp(__double2float_rn(d)), 1.f), 1.f); /* 0/0: 1 */
+    const float m = fminf(__fmaf_rn(__double2float_rn(n), frcp(__double2float_rn(d)), 1.f), 0x1p126f);
     const int b = (__float_as_int(m) + 0x10000) & 0x7ffe0000;
     const double c = widen(b);
     const double e = sub(__hiloint2double(0x43300000, (b >> 23) - 127), 4503599627370496.);
