@@ -38,12 +38,12 @@ __device__ __forceinline__ void eval_chunk64(const void *staged, int count, cons
             for (; h < count; h++) ex::hess_pairs<TYPE, P, 1>(r + h, px, py, acc.run);
         return;
     }
-    /* the chunk's sums, which join the totals once: one running sum of all halos rounds at the
-     * size of the total with every halo (convergence of 700 halos 7.6e-16 off, 5.3e-16 as two
-     * diagonal entries) */
-    double gx[P], gy[P], ka[P], g1[P], g2[P], psi[P];
+    /* the chunk's convergence, which joins the total once: its terms have one sign, and one running
+     * sum of all halos rounds at the size of the total with every halo (convergence of 700 halos
+     * 7.6e-16 off, 5.3e-16 as two diagonal entries) */
+    double ka[P];
 #pragma unroll
-    for (int k = 0; k < P; k++) gx[k] = gy[k] = ka[k] = g1[k] = g2[k] = psi[k] = 0.;
+    for (int k = 0; k < P; k++) ka[k] = 0.;
 #pragma unroll 1
     for (int h = 0; h < count; h++) {
         const lt_nie64 &r = static_cast<const lt_nie64 *>(staged)[h];
@@ -51,23 +51,14 @@ __device__ __forceinline__ void eval_chunk64(const void *staged, int count, cons
 #pragma unroll
         for (int k = 0; k < P; k++) {
             const Nie64 n = nie64<TYPE>(r, px[k], py);
-            if (OP & OP_GRAD) grad_nie<TYPE>(r, n, gx[k], gy[k]);
-            if (OP & OP_HESS) kg_nie<TYPE>(r, n, w, ka[k], g1[k], g2[k]);
-            if (OP & OP_POT) pot_nie<TYPE>(r, n, psi[k]);
+            if (OP & OP_GRAD) grad_nie<TYPE>(r, n, acc.gx[k], acc.gy[k]);
+            if (OP & OP_HESS) kg_nie<TYPE>(r, n, w, ka[k], acc.hyy[k], acc.hxy[k]);
+            if (OP & OP_POT) pot_nie<TYPE>(r, n, acc.psi[k]);
         }
     }
+    if (OP & OP_HESS) {
 #pragma unroll
-    for (int k = 0; k < P; k++) {
-        if (OP & OP_GRAD) {
-            acc.gx[k] = c64::add(acc.gx[k], gx[k]);
-            acc.gy[k] = c64::add(acc.gy[k], gy[k]);
-        }
-        if (OP & OP_HESS) {
-            acc.hxx[k] = c64::add(acc.hxx[k], ka[k]);
-            acc.hyy[k] = c64::add(acc.hyy[k], g1[k]);
-            acc.hxy[k] = c64::add(acc.hxy[k], g2[k]);
-        }
-        if (OP & OP_POT) acc.psi[k] = c64::add(acc.psi[k], psi[k]);
+        for (int k = 0; k < P; k++) acc.hxx[k] = c64::add(acc.hxx[k], ka[k]);
     }
 }
 
