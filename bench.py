@@ -62,7 +62,7 @@ FLOPS_PER_PAIR = 182 + 760
 # hash to INST_SOURCES_SHA; the bench line says whether the timed build is that one.
 KERNEL_SOURCES = ("lt_eval.cuh", "lt_profiles32.cuh", "lt_profiles64.cuh", "lt_bulk.cuh", "lt_grid32.cu",
                   "lt_closed64.cuh", "lt_grid.cuh", "lt_halo.h", "lt_pack.h")
-INST_SOURCES_SHA = "a711fb3c92f4d232"
+INST_SOURCES_SHA = "4ba8af0b7c912cd5"
 INST_PER_PAIR_FP32C_LENS = 100.2
 FP32_FLOPS_PER_PAIR_FP32C_LENS = 126.4
 # DRAM bytes (read + write) of one launch of that kernel at 4096^2, from a single-pass ncu
